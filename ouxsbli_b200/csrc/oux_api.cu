@@ -145,6 +145,17 @@ int visc_kind_base(const oux_config* c, std::string& why) {
   return -1;
 }
 
+// delta^(3/2) of the SGS model (calc_les.f90:62-68) from the inverse spacings of a grid
+// of uniform spacings.
+double sms_delta15_host(const oux_config& c) {
+  const double ix = 1.0 / c.dx[0], iy = 1.0 / c.dy[0], iz = 1.0 / c.dz[0];
+  const double mn = std::min(std::min(ix, iy), iz);
+  const double l1 = std::log(mn / ix), l2 = std::log(mn / iy);
+  const double delta =
+      std::cosh(std::sqrt(4.0 * (l1 * l1 - l1 * l2 + l2 * l2) / 27.0)) * std::pow(ix * iy * iz, -1.0 / 3.0);
+  return delta * std::sqrt(delta);
+}
+
 void build_tables(oux_handle* h) {
   const oux_config& c = h->cfg;
   const double* dx = c.dx;
@@ -207,6 +218,7 @@ void build_tables(oux_handle* h) {
   K.T_ref = 0.0;
   double t10 = std::tan(10.0 * std::acos(-1.0) / 180.0);
   K.tan10deg2 = t10 * t10;
+  K.delta15 = c.visc == OUX_LES && h->G.uni == 7 ? sms_delta15_host(c) : 0.0;
 }
 
 Geo make_geo(const oux_config& c) {
@@ -518,8 +530,8 @@ int launch_prim_fused(const TQ* q, const TS* src, const Geo& G, Fields<T>& W, ou
   if constexpr (MX) {
     if (!std::is_same<TS, double>::value) inc = reinterpret_cast<const float*>(src);
   }
-  constexpr size_t smem = prim_fused_smem<1>();
-  auto kern = k_prim_fused<1, true, VISC, MX, TQ, T>;
+  constexpr size_t smem = prim_fused_smem();
+  auto kern = k_prim_fused<VISC, MX, TQ, T>;
   static const cudaError_t attr = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (attr != cudaSuccess) return 1;
   kern<<<prim_fused_grid(G), PS_TX * PS_TY, smem, s>>>(q, inc, G, W, h->M, h->K);
@@ -533,7 +545,6 @@ int run_stage(oux_handle* h, const TS* src, StepArgs<T> A, cudaStream_t s) {
   const Geo& G = h->G;
   const oux_config& c = h->cfg;
   Fields<T>& W = fields_of<T>(h);
-  int64_t ncell = (int64_t)G.nx * G.ny * G.nz;
   bool visc = c.visc != OUX_EULER;
   const bool sens = c.scheme != OUX_KEEP;
   // FP64 with gradient fields: the plain primitive pass, and the sensor in the gradient
@@ -602,16 +613,13 @@ int run_stage(oux_handle* h, const TS* src, StepArgs<T> A, cudaStream_t s) {
     }
   }
   if (h->les) {
-    dim3 b(32, 4, 1), gr((G.nx - 2 + 31) / 32, (G.ny - 2 + 3) / 4, G.nz - 2);
-    {
-      Timed tm(h, KK_MUT, s);
-      k_mut<T><<<gr, b, 0, s>>>(G, W, h->M, h->K);
-    }
-    {
-      Timed tm(h, KK_MUT_EDGES, s);
-      k_mut_edges<T><<<grid_for(ncell, 256), 256, 0, s>>>(G, W);
-    }
-    h->launches += 2;
+    Timed tm(h, KK_MUT, s);
+    constexpr size_t smem = mut_smem<T>();
+    static const cudaError_t attr =
+        cudaFuncSetAttribute(k_mut<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (attr != cudaSuccess) return fail(OUX_E_CUDA, "SGS viscosity pass: shared memory");
+    k_mut<T><<<mut_grid(G), MUT_TX * MUT_TY, smem, s>>>(G, W, h->M, h->K);
+    h->launches++;
   }
   int rc;
   if (h->profiling) {
@@ -892,6 +900,7 @@ PhysConst consts_of(const oux_config& c) {
   K.T_ref = 0.0;
   double t10 = std::tan(10.0 * std::acos(-1.0) / 180.0);
   K.tan10deg2 = t10 * t10;
+  K.delta15 = c.visc == OUX_LES && make_geo(c).uni == 7 ? sms_delta15_host(c) : 0.0;
   return K;
 }
 

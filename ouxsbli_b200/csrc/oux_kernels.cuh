@@ -137,29 +137,38 @@ inline dim3 plane_grid(const Geo& G) {
 }
 
 // ---- prim: src/calc_physical_quantities.f90:60-116 (3D), :7-57 (2D) -------
+// The primitive fields of a cell from its FP64 conservative values q (mixed form MX: p
+// and T stored as deviations from K.p_ref, K.T_ref, everything rounded once); v returns
+// the velocities in FP64.
+template <int DIM, bool VISC, bool MX, class T>
+__device__ __forceinline__ void prim_store(const double* q, double Jv, const Fields<T>& W, int64_t o,
+                                           const PhysConst& K, double (&v)[3]) {
+  const double over = 1.0 / q[0], rho = Jv * q[0];
+  v[0] = q[1] * over;
+  v[1] = q[2] * over;
+  v[2] = DIM == 3 ? q[3] * over : 0.0;
+  double p;
+  if constexpr (DIM == 3) p = K.gamma_1 * (Jv * q[4] - 0.5 * rho * (v[0] * v[0] + v[1] * v[1] + v[2] * v[2]));
+  else p = K.gamma_1 * (Jv * q[3] - 0.5 * rho * (v[0] * v[0] + v[1] * v[1]));
+  const double temp = p / (K.R * rho);
+  W.rho[o] = (T)rho;
+  W.u[o] = (T)v[0];
+  W.v[o] = (T)v[1];
+  if constexpr (DIM == 3) W.w[o] = (T)v[2];
+  W.p[o] = MX ? (T)(p - K.p_ref) : (T)p;
+  W.T_[o] = MX ? (T)(temp - K.T_ref) : (T)temp;
+  if constexpr (VISC) W.mu[o] = (T)(K.sutherland / (temp + 111.0) * (temp * sqrt(temp)));
+}
+
 template <int DIM, bool VISC, class TS, class T, bool RO = false>
 __device__ __forceinline__ void prim_cell(const TS* Q, const Geo& G, const Fields<T>& W, const double* jac,
                                           const PhysConst& K, int i, int j, int k) {
-  int64_t o = G.at(i, j, k);
-  T Jv = (T)ldro<RO>(jac + (int64_t)j * G.nx + i);
-  T q1 = (T)ldro<RO>(Q + o);
-  T over_Q1 = T(1) / q1;
-  T rho = Jv * q1;
-  T u = (T)ldro<RO>(Q + o + G.vs) * over_Q1;
-  T v = (T)ldro<RO>(Q + o + 2 * G.vs) * over_Q1;
-  T w = T(0), p;
-  if constexpr (DIM == 3) {
-    w = (T)ldro<RO>(Q + o + 3 * G.vs) * over_Q1;
-    p = T(K.gamma_1) * (Jv * (T)ldro<RO>(Q + o + 4 * G.vs) - T(0.5) * rho * (u * u + v * v + w * w));
-  } else {
-    p = T(K.gamma_1) * (Jv * (T)ldro<RO>(Q + o + 3 * G.vs) - T(0.5) * rho * (u * u + v * v));
-  }
-  W.rho[o] = rho; W.u[o] = u; W.v[o] = v;
-  if constexpr (DIM == 3) W.w[o] = w;
-  W.p[o] = p;
-  T temp = p / (T(K.R) * rho);
-  W.T_[o] = temp;
-  if constexpr (VISC) W.mu[o] = T(K.sutherland) / (temp + T(111)) * (temp * sqrt(temp));
+  static_assert(sizeof(T) == sizeof(double), "the mixed form decodes through prim_mx_cell");
+  const int64_t o = G.at(i, j, k);
+  double q[DIM + 2], v[3];
+#pragma unroll
+  for (int l = 0; l < DIM + 2; ++l) q[l] = (double)ldro<RO>(Q + o + l * G.vs);
+  prim_store<DIM, VISC, false>(q, ldro<RO>(jac + (int64_t)j * G.nx + i), W, o, K, v);
 }
 
 template <int DIM, bool VISC, class TS, class T, bool RO = false>
@@ -189,21 +198,8 @@ __device__ __forceinline__ void prim_mx_cell(const double* Qn, const float* dQ, 
 #pragma unroll
   for (int l = 0; l < DIM + 2; ++l)
     q[l] = ldro<RO>(Qn + o + l * G.vs) + (dQ ? (double)ldro<RO>(dQ + o + l * G.vs) : 0.0);
-  double Jv = ldro<RO>(jac + (int64_t)j * G.nx + i);
-  double over = 1.0 / q[0], rho = Jv * q[0];
-  double u = q[1] * over, v = q[2] * over, w = 0.0, p;
-  if constexpr (DIM == 3) {
-    w = q[3] * over;
-    p = K.gamma_1 * (Jv * q[4] - 0.5 * rho * (u * u + v * v + w * w));
-  } else {
-    p = K.gamma_1 * (Jv * q[3] - 0.5 * rho * (u * u + v * v));
-  }
-  double temp = p / (K.R * rho);
-  W.rho[o] = (float)rho; W.u[o] = (float)u; W.v[o] = (float)v;
-  if constexpr (DIM == 3) W.w[o] = (float)w;
-  W.p[o] = (float)(p - K.p_ref);
-  W.T_[o] = (float)(temp - K.T_ref);
-  if constexpr (VISC) W.mu[o] = (float)(K.sutherland / (temp + 111.0) * (temp * sqrt(temp)));
+  double v[3];
+  prim_store<DIM, VISC, true>(q, ldro<RO>(jac + (int64_t)j * G.nx + i), W, o, K, v);
 }
 
 template <int DIM, bool VISC, bool RO = false>
@@ -383,111 +379,90 @@ __global__ void __launch_bounds__(PLANE_THREADS) k_sensor_mx(Geo G, const double
 }
 
 // ---- primitives and Ducros sensor in one pass (3D) --------------------------------
-// A block owns a PS_TX x PS_TY column of cells (x, y) over PS_PLANES z planes and
-// marches along z.  For every plane it decodes the velocities of its cells and of a
-// one-cell ring around them into shared memory (the last three planes are kept),
-// writes its own cells' primitive fields (prim_cell / prim_mx_cell), and evaluates the
-// previous plane's sensor from shared memory with the FP64 sensor's arithmetic
+// A block owns PS_TX x PS_TY x PS_TZ cells.  It decodes the velocities of its cells and
+// of a one-cell ring around them into shared memory, writing its own cells' primitive
+// fields on the way (prim_cell / prim_mx_cell on the same loads), and after one barrier
+// evaluates its cells' sensors from shared memory with the FP64 sensor's arithmetic
 // (calc_Ducros, 3D_solver/src/calc_hybrid.f90:11-72, with the reference's copies to
-// the outer faces).  Q is read once per cell plus the ring (mostly from L2), and the
-// sensor's neighbour velocities never leave the SM.
+// the outer faces).  The ring re-reads 2x of the momenta, from L2.
 //   FP64 form: the same bits as k_prim then k_sensor (the same expressions on the
 //   same values).
 //   Mixed form (MX): velocities decoded in FP64 from Q^n + the FP32 increment dQ, so
 //   the sensor is sensor_mx_cell's value, rounded once when stored.
-constexpr int PS_TX = 32, PS_TY = 8, PS_PLANES = 32;
+// Bound: load latency, then HBM (92 B per cell in the mixed viscous form).  Every load
+// of the tile is independent, and a grid gives 8x more blocks than one that marches a
+// column over 32 planes with two barriers a plane, which left 38^3 to 134^3 grids on 20
+// to 340 blocks: mixed, us per launch, 38^3 82 -> 16, 87^3 100 -> 32, 134^3 124 -> 85,
+// 262^3 536 -> 521.  PS_TZ 2 / 4 / 8 at 262^3: 609 / 521 / 768 (ring re-reads against
+// resident blocks); one cell in flight a thread at 4 blocks per SM beats two at 3 (831).
+constexpr int PS_TX = 32, PS_TY = 8, PS_TZ = 4;
 
-template <int HD> __host__ __device__ constexpr size_t prim_fused_smem() {
-  return sizeof(double) * (2 * HD + 1) * 3 * (PS_TY + 2 * HD) * (PS_TX + 2 * HD);
+constexpr size_t prim_fused_smem() {
+  return sizeof(double) * 3 * (PS_TZ + 2) * (PS_TY + 2) * (PS_TX + 2);
 }
 
 inline dim3 prim_fused_grid(const Geo& G) {
   return dim3((unsigned)((G.nx + PS_TX - 1) / PS_TX), (unsigned)((G.ny + PS_TY - 1) / PS_TY),
-              (unsigned)((G.pk1 - G.pk0 + PS_PLANES - 1) / PS_PLANES));
+              (unsigned)((G.pk1 - G.pk0 + PS_TZ - 1) / PS_TZ));
 }
 
-template <int HD, bool SENSOR, bool VISC, bool MX, class TS, class T>
-__global__ void __launch_bounds__(PS_TX * PS_TY) k_prim_fused(const TS* __restrict__ Q, const float* __restrict__ dQ,
+template <bool VISC, bool MX, class TS, class T>
+__global__ void __launch_bounds__(PS_TX * PS_TY, 4) k_prim_fused(const TS* __restrict__ Q, const float* __restrict__ dQ,
                                                               Geo G, Fields<T> W, Metrics M, PhysConst K) {
-  static_assert(HD == 1, "the sensor's ring is one cell wide");
-  constexpr int NW = 2 * HD + 1;                      // planes kept
-  constexpr int RX = PS_TX + 2 * HD, RY = PS_TY + 2 * HD;
+  constexpr int RX = PS_TX + 2, RY = PS_TY + 2, RZ = PS_TZ + 2, RN = RX * RY * RZ;
   extern __shared__ __align__(16) unsigned char smraw[];
-  double* vel = reinterpret_cast<double*>(smraw);     // [plane slot][component][ry][rx]
-  auto V = [&](int slot, int c, int y, int x) -> double& { return vel[((slot * 3 + c) * RY + y) * RX + x]; };
+  double* vel = reinterpret_cast<double*>(smraw);  // [component][rz][ry][rx]
   const int tid = threadIdx.x;
   const int bx = blockIdx.x * PS_TX, by = blockIdx.y * PS_TY;
-  const int k0 = G.pk0 + blockIdx.z * PS_PLANES, k1 = min(G.pk1, k0 + PS_PLANES);
+  const int k0 = G.pk0 + blockIdx.z * PS_TZ, k1 = min(G.pk1, k0 + PS_TZ);
+#pragma unroll 1
+  for (int c = tid; c < RN; c += PS_TX * PS_TY) {
+    const int cx = c % RX, r = c / RX, cy = r % RY, cz = r / RY;
+    const int i = bx - 1 + cx, j = by - 1 + cy, k = k0 - 1 + cz;
+    if (i < 0 || i >= G.nx || j < 0 || j >= G.ny || k < 0 || k >= G.nz || k > k1) continue;
+    const int64_t o = G.at(i, j, k);
+    double q[5];
+    const bool own = cx >= 1 && cx <= PS_TX && cy >= 1 && cy <= PS_TY && k >= k0 && k < k1;
+#pragma unroll
+    for (int l = 0; l < 5; ++l) {
+      if (l == 4 && !own) break;
+      q[l] = (double)__ldg(Q + o + l * G.vs);
+      if constexpr (MX) q[l] = q[l] + (dQ ? (double)__ldg(dQ + o + l * G.vs) : 0.0);
+    }
+    double v[3];
+    if (own) {
+      prim_store<3, VISC, MX>(q, __ldg(M.jac + (int64_t)j * G.nx + i), W, o, K, v);
+    } else {
+      const double over = 1.0 / q[0];
+      v[0] = q[1] * over;
+      v[1] = q[2] * over;
+      v[2] = q[3] * over;
+    }
+    vel[c] = v[0];
+    vel[RN + c] = v[1];
+    vel[2 * RN + c] = v[2];
+  }
+  __syncthreads();
   const int tx = tid % PS_TX, ty = tid / PS_TX;
-  const int oi = bx + tx, oj = by + ty;  // this thread's own cell
-  const bool own = oi < G.nx && oj < G.ny;
-  const int rx = tx + HD, ry = ty + HD;  // and its place in the ring
-  auto slot_of = [](int k) { return (k % NW + NW) % NW; };
-  for (int kk = k0 - HD; kk < k1 + HD; ++kk) {
-    // 1. velocities of plane kk (block cells and ring)
-    if (kk >= 0 && kk < G.nz) {
-      const int slot = slot_of(kk);
-      for (int c = tid; c < RX * RY; c += PS_TX * PS_TY) {
-        const int cx = c % RX, cy = c / RX;
-        const int i = bx - HD + cx, j = by - HD + cy;
-        if (i < 0 || i >= G.nx || j < 0 || j >= G.ny) continue;
-        const int64_t o = G.at(i, j, kk);
-        double q0, q1, q2, q3;
-        if constexpr (MX) {
-          const double* Qd = reinterpret_cast<const double*>(Q);
-          q0 = __ldg(Qd + o) + (dQ ? (double)__ldg(dQ + o) : 0.0);
-          q1 = __ldg(Qd + o + G.vs) + (dQ ? (double)__ldg(dQ + o + G.vs) : 0.0);
-          q2 = __ldg(Qd + o + 2 * G.vs) + (dQ ? (double)__ldg(dQ + o + 2 * G.vs) : 0.0);
-          q3 = __ldg(Qd + o + 3 * G.vs) + (dQ ? (double)__ldg(dQ + o + 3 * G.vs) : 0.0);
-        } else {
-          q0 = (double)__ldg(Q + o);
-          q1 = (double)__ldg(Q + o + G.vs);
-          q2 = (double)__ldg(Q + o + 2 * G.vs);
-          q3 = (double)__ldg(Q + o + 3 * G.vs);
-        }
-        const double over = 1.0 / q0;  // prim_cell / prim_mx_cell: u = q1 * (1 / q0)
-        V(slot, 0, cy, cx) = q1 * over;
-        V(slot, 1, cy, cx) = q2 * over;
-        V(slot, 2, cy, cx) = q3 * over;
-      }
-      // 2. the block's own cells: every primitive field
-      if (own && kk >= k0 && kk < k1) {
-        if constexpr (MX) prim_mx_cell<3, VISC, true>(reinterpret_cast<const double*>(Q), dQ, G, W, M.jac, K, oi, oj, kk);
-        else prim_cell<3, VISC, TS, T, true>(Q, G, W, M.jac, K, oi, oj, kk);
-      }
-    }
-    __syncthreads();
-    // 3. the sensor of plane k = kk - 1 from the planes k - 1, k, k + 1
-    if constexpr (SENSOR) {
-      const int k = kk - 1;
-      if (own && k >= k0 && k < k1 && oi >= 1 && oi <= G.nx - 2 && oj >= 1 && oj <= G.ny - 2 && k >= 1 &&
-          k <= G.nz - 2) {
-        const int sm = slot_of(k - 1), s0 = slot_of(k), sp = slot_of(k + 1);
-        const double dxt = 0.25 * (M.inv_dx[oi - 1] + M.inv_dx[oi]);
-        const double dyt = 0.25 * (M.inv_dy[oj - 1] + M.inv_dy[oj]);
-        const double dzt = 0.25 * (M.inv_dz[k - 1] + M.inv_dz[k]);
-        const double dudx = (-V(s0, 0, ry, rx - 1) + V(s0, 0, ry, rx + 1)) * dxt;
-        const double dvdx = (-V(s0, 1, ry, rx - 1) + V(s0, 1, ry, rx + 1)) * dxt;
-        const double dwdx = (-V(s0, 2, ry, rx - 1) + V(s0, 2, ry, rx + 1)) * dxt;
-        const double dudy = (-V(s0, 0, ry - 1, rx) + V(s0, 0, ry + 1, rx)) * dyt;
-        const double dvdy = (-V(s0, 1, ry - 1, rx) + V(s0, 1, ry + 1, rx)) * dyt;
-        const double dwdy = (-V(s0, 2, ry - 1, rx) + V(s0, 2, ry + 1, rx)) * dyt;
-        const double dudz = (-V(sm, 0, ry, rx) + V(sp, 0, ry, rx)) * dzt;
-        const double dvdz = (-V(sm, 1, ry, rx) + V(sp, 1, ry, rx)) * dzt;
-        const double dwdz = (-V(sm, 2, ry, rx) + V(sp, 2, ry, rx)) * dzt;
-        const double div = dudx + dvdy + dwdz;
-        const double r1 = dwdy - dvdz, r2 = dudz - dwdx, r3 = dvdx - dudy;
-        double f = (div * div) / (div * div + (r1 * r1 + r2 * r2 + r3 * r3) + 1.0e-12);
-        f = fmin_f(1.0, f);
-        const T fs = (T)f;
-        const int i = oi, j = oj;
-        W.sensor[G.at(i, j, k)] = fs;
-        if (i == 1) W.sensor[G.at(0, j, k)] = fs; else if (i == G.nx - 2) W.sensor[G.at(G.nx - 1, j, k)] = fs;
-        if (j == 1) W.sensor[G.at(i, 0, k)] = fs; else if (j == G.ny - 2) W.sensor[G.at(i, G.ny - 1, k)] = fs;
-        if (k == 1) W.sensor[G.at(i, j, 0)] = fs; else if (k == G.nz - 2) W.sensor[G.at(i, j, G.nz - 1)] = fs;
-      }
-    }
-    __syncthreads();
+  const int i = bx + tx, j = by + ty;
+  if (i < 1 || i > G.nx - 2 || j < 1 || j > G.ny - 2) return;
+  const double dxt = 0.25 * (M.inv_dx[i - 1] + M.inv_dx[i]);
+  const double dyt = 0.25 * (M.inv_dy[j - 1] + M.inv_dy[j]);
+  for (int k = max(k0, 1); k < min(k1, G.nz - 1); ++k) {
+    const double dzt = 0.25 * (M.inv_dz[k - 1] + M.inv_dz[k]);
+    const double* V = vel + ((k - k0 + 1) * RY + ty + 1) * RX + tx + 1;
+    auto df = [&](int c, int st) -> double { return -V[c * RN - st] + V[c * RN + st]; };
+    const double dudx = df(0, 1) * dxt, dvdx = df(1, 1) * dxt, dwdx = df(2, 1) * dxt;
+    const double dudy = df(0, RX) * dyt, dvdy = df(1, RX) * dyt, dwdy = df(2, RX) * dyt;
+    const double dudz = df(0, RX * RY) * dzt, dvdz = df(1, RX * RY) * dzt, dwdz = df(2, RX * RY) * dzt;
+    const double div = dudx + dvdy + dwdz;
+    const double r1 = dwdy - dvdz, r2 = dudz - dwdx, r3 = dvdx - dudy;
+    double f = (div * div) / (div * div + (r1 * r1 + r2 * r2 + r3 * r3) + 1.0e-12);
+    const T fs = (T)fmin_f(1.0, f);
+    W.sensor[G.at(i, j, k)] = fs;
+    if (i == 1) W.sensor[G.at(0, j, k)] = fs; else if (i == G.nx - 2) W.sensor[G.at(G.nx - 1, j, k)] = fs;
+    if (j == 1) W.sensor[G.at(i, 0, k)] = fs; else if (j == G.ny - 2) W.sensor[G.at(i, G.ny - 1, k)] = fs;
+    if (k == 1) W.sensor[G.at(i, j, 0)] = fs; else if (k == G.nz - 2) W.sensor[G.at(i, j, G.nz - 1)] = fs;
   }
 }
 
@@ -576,87 +551,184 @@ __global__ void __launch_bounds__(PLANE_THREADS, 8) k_grad(Geo G, Fields<T> W, M
 
 // ---- SMS sub-grid model: 3D_solver/src/calc_les.f90:30-125 -------------------
 template <class T>
-__device__ __forceinline__ void grad3(const T (&u)[3][3][3], const T (&v)[3][3][3], const T (&w)[3][3][3],
-                                      T dx, T dy, T dz, T d[9]) {  // calc_differential :11-27
-  d[0] = T(0.5) * (-u[1][1][0] + u[1][1][2]) * dx;
-  d[1] = T(0.5) * (-u[1][0][1] + u[1][2][1]) * dy;
-  d[2] = T(0.5) * (-u[0][1][1] + u[2][1][1]) * dz;
-  d[3] = T(0.5) * (-v[1][1][0] + v[1][1][2]) * dx;
-  d[4] = T(0.5) * (-v[1][0][1] + v[1][2][1]) * dy;
-  d[5] = T(0.5) * (-v[0][1][1] + v[2][1][1]) * dz;
-  d[6] = T(0.5) * (-w[1][1][0] + w[1][1][2]) * dx;
-  d[7] = T(0.5) * (-w[1][0][1] + w[1][2][1]) * dy;
-  d[8] = T(0.5) * (-w[0][1][1] + w[2][1][1]) * dz;
-}
-
-template <class T>
 __device__ __forceinline__ T filt(const T* a, int64_t o, int64_t sx, int64_t pl) {  // test_filter :74-80
   T c = a[o];
   return c + T(0.25) * (a[o - 1] - T(2) * c + a[o + 1] + a[o - sx] - T(2) * c + a[o + sx] + a[o - pl] -
                         T(2) * c + a[o + pl]);
 }
 
-// One cell (i, j, k) of calc_mut, 1 <= i,j,k <= n-2.
+// SMS :30-71 of one cell: SGS viscosity from the velocity gradients a[3c + axis], the
+// vorticity vh of the test-filtered field, the filtered-out kinetic energy qc2 and
+// delta15 = delta^(3/2).  S2^(1/4) and qc2^(1/4) are square roots of square roots
+// (correctly rounded each, where pow is within an ulp or two).
 template <class T>
-__device__ __forceinline__ void mut_cell(const Geo& G, const Fields<T>& W, const Metrics& M, const PhysConst& K,
-                                         int i, int j, int k) {
-  const int64_t sx = G.sx, pl = G.plane;
-  int64_t o = G.at(i, j, k);
-  T u3[3][3][3], v3[3][3][3], w3[3][3][3], ut[3][3][3], vt[3][3][3], wt[3][3][3];
-  bool inner = (2 <= i && i <= G.nx - 3 && 2 <= j && j <= G.ny - 3 && 2 <= k && k <= G.nz - 3);
-#pragma unroll
-  for (int c = 0; c < 3; ++c)
-#pragma unroll
-    for (int b = 0; b < 3; ++b)
-#pragma unroll
-      for (int a = 0; a < 3; ++a) {
-        int64_t q = o + (a - 1) + (b - 1) * sx + (c - 1) * pl;
-        u3[c][b][a] = W.u[q]; v3[c][b][a] = W.v[q]; w3[c][b][a] = W.w[q];
-        if (inner) {
-          ut[c][b][a] = filt(W.u, q, sx, pl);
-          vt[c][b][a] = filt(W.v, q, sx, pl);
-          wt[c][b][a] = filt(W.w, q, sx, pl);
-        } else {
-          ut[c][b][a] = u3[c][b][a]; vt[c][b][a] = v3[c][b][a]; wt[c][b][a] = w3[c][b][a];
-        }
-      }
-  T du = u3[1][1][1] - ut[1][1][1], dv = v3[1][1][1] - vt[1][1][1], dw = w3[1][1][1] - wt[1][1][1];
-  T qc2 = T(0.5) * (du * du + dv * dv + dw * dw);
-  // SMS :30-71
-  T dx = (T)M.inv_dx[i], dy = (T)M.inv_dy[j], dz = (T)M.inv_dz[k];
-  T a[9], h[9];
-  grad3(u3, v3, w3, dx, dy, dz, a);
-  grad3(ut, vt, wt, dx, dy, dz, h);
+__device__ __forceinline__ T sms_mut(const T a[9], T vh1, T vh2, T vh3, T qc2, T rho, T delta15, T tan10deg2) {
   T vo1 = a[7] - a[5], vo2 = a[2] - a[6], vo3 = a[3] - a[1];
-  T vh1 = h[7] - h[5], vh2 = h[2] - h[6], vh3 = h[3] - h[1];
   T vd1 = vo1 - vh1, vd2 = vo2 - vh2, vd3 = vo3 - vh3;
   T vor2 = vo1 * vo1 + vo2 * vo2 + vo3 * vo3;
   T vorh2 = vh1 * vh1 + vh2 * vh2 + vh3 * vh3;
   T vdif2 = vd1 * vd1 + vd2 * vd2 + vd3 * vd3;
-  T svor2 = T(2) * sqrt(vor2) * sqrt(vorh2) + vorh2 + vor2 - vdif2;
-  T tan2 = (fabs(svor2) < T(1.0e-30)) ? T(0)
-                                       : (T(2) * sqrt(vorh2) * sqrt(vor2) - vorh2 - vor2 + vdif2) / svor2;
-  T rth = tan2 / T(K.tan10deg2);
+  T svor = sqrt(vor2), svorh = sqrt(vorh2);
+  T svor2 = T(2) * svor * svorh + vorh2 + vor2 - vdif2;
+  T tan2 = (fabs(svor2) < T(1.0e-30)) ? T(0) : (T(2) * svorh * svor - vorh2 - vor2 + vdif2) / svor2;
+  T rth = tan2 / tan10deg2;
   T fth = fmin_f(T(1), rth * rth);
   T S2 = T(2) * (a[0] * a[0] + a[4] * a[4] + a[8] * a[8]) +
          ((a[3] + a[1]) * (a[3] + a[1]) + (a[7] + a[5]) * (a[7] + a[5]) + (a[2] + a[6]) * (a[2] + a[6]));
-  T mn = fmin_f(fmin_f(dx, dy), dz);
-  T a1 = mn / dx, a2 = mn / dy;
-  T l1 = log(a1), l2 = log(a2);
-  T delta = cosh(sqrt(T(4) * (l1 * l1 - l1 * l2 + l2 * l2) / T(27))) * pow(dx * dy * dz, T(-1.0 / 3.0));
-  const T Cm = T(0.06), alpha = T(0.5);
-  T nut = fth * Cm * pow(S2, T(0.5) * alpha) * pow(qc2, T(0.5) * (T(1) - alpha)) * pow(delta, T(1) + alpha);
+  const T Cm = T(0.06);
+  T nut = fth * Cm * sqrt(sqrt(S2)) * sqrt(sqrt(qc2)) * delta15;
+  return rho * nut;
+}
+
+// delta^(3/2) of the cell: K.delta15 on grids whose spacings are the same on every axis
+// (the host evaluates it once: log, cosh and pow per cell were half of the pass's
+// instructions), else from the cell's inverse spacings.
+template <class T>
+__device__ __forceinline__ T sms_delta15(const Geo& G, const Metrics& M, const PhysConst& K, int i, int j, int k) {
+  if (G.uni == 7) return T(K.delta15);
+  const T dx = (T)M.inv_dx[i], dy = (T)M.inv_dy[j], dz = (T)M.inv_dz[k];
+  const T mn = fmin_f(fmin_f(dx, dy), dz);
+  const T l1 = log(mn / dx), l2 = log(mn / dy);
+  const T delta = cosh(sqrt(T(4) * (l1 * l1 - l1 * l2 + l2 * l2) / T(27))) * pow(dx * dy * dz, T(-1.0 / 3.0));
+  return delta * sqrt(delta);
+}
+
+// Cells 2 <= i,j,k <= n-3 take the test-filtered field; the others the field itself.
+__device__ __forceinline__ bool mut_inner(const Geo& G, int i, int j, int k) {
+  return 2 <= i && i <= G.nx - 3 && 2 <= j && j <= G.ny - 3 && 2 <= k && k <= G.nz - 3;
+}
+
+// One cell (i, j, k) of calc_mut, 1 <= i,j,k <= n-2 (the batched kernel; k_mut shares
+// the filtered field of a tile).
+template <class T>
+__device__ __forceinline__ void mut_cell(const Geo& G, const Fields<T>& W, const Metrics& M, const PhysConst& K,
+                                         int i, int j, int k) {
+  const int64_t st[3] = {1, G.sx, G.plane};
+  const int64_t o = G.at(i, j, k);
+  const T* vel[3] = {W.u, W.v, W.w};
+  const T inv[3] = {(T)M.inv_dx[i], (T)M.inv_dy[j], (T)M.inv_dz[k]};
+  const bool inner = mut_inner(G, i, j, k);
+  T a[9], h[9], qc2 = T(0);
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      const T* f = vel[c];
+      a[3 * c + d] = T(0.5) * (-f[o - st[d]] + f[o + st[d]]) * inv[d];
+      h[3 * c + d] = a[3 * c + d];
+      if (inner && c != d)
+        h[3 * c + d] =
+            T(0.5) * (-filt(f, o - st[d], G.sx, G.plane) + filt(f, o + st[d], G.sx, G.plane)) * inv[d];
+    }
+    const T dv = inner ? vel[c][o] - filt(vel[c], o, G.sx, G.plane) : T(0);
+    qc2 = c == 0 ? dv * dv : qc2 + dv * dv;
+  }
+  qc2 = T(0.5) * qc2;
   W.qc2[o] = qc2;
-  W.mut[o] = W.rho[o] * nut;
+  W.mut[o] = sms_mut<T>(a, h[7] - h[5], h[2] - h[6], h[3] - h[1], qc2, W.rho[o], sms_delta15<T>(G, M, K, i, j, k),
+                        T(K.tan10deg2));
+}
+
+// SGS viscosity and q_c^2 of cells 1 .. n-2, and of the edge cells (mut_edge_cell's rule,
+// written by the thread that owns their source cell).  A block owns MUT_TX x MUT_TY x
+// MUT_TZ cells and filters the velocities of its cells and a one-cell ring once into
+// shared memory.  Bound: instruction issue (square roots and divisions) and L1.
+// Measured in the mixed form, with the edge pass it replaces (us per stage): 38^3
+// 17.3 -> 14.9, 87^3 45.8 -> 31.1, 134^3 134 -> 79; MUT_TZ 2 / 4 / 8 at 134^3: 85 / 79 / 78.
+constexpr int MUT_TX = 32, MUT_TY = 8, MUT_TZ = 4;
+template <class T> constexpr size_t mut_smem() {
+  return sizeof(T) * 3 * (MUT_TX + 2) * (MUT_TY + 2) * (MUT_TZ + 2);
+}
+inline dim3 mut_grid(const Geo& G) {
+  return dim3((unsigned)((G.nx - 2 + MUT_TX - 1) / MUT_TX), (unsigned)((G.ny - 2 + MUT_TY - 1) / MUT_TY),
+              (unsigned)((G.nz - 2 + MUT_TZ - 1) / MUT_TZ));
 }
 
 template <class T>
-__global__ void k_mut(Geo G, Fields<T> W, Metrics M, PhysConst K) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
-  int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
-  int k = blockIdx.z * blockDim.z + threadIdx.z + 1;
-  if (i > G.nx - 2 || j > G.ny - 2 || k > G.nz - 2) return;
-  mut_cell<T>(G, W, M, K, i, j, k);
+__global__ void __launch_bounds__(MUT_TX * MUT_TY) k_mut(Geo G, Fields<T> W, Metrics M, PhysConst K) {
+  constexpr int RX = MUT_TX + 2, RY = MUT_TY + 2, RZ = MUT_TZ + 2, RN = RX * RY * RZ;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  T* fv = reinterpret_cast<T*>(smraw);  // filtered velocity [component][rz][ry][rx]
+  const int tid = threadIdx.x;
+  const int bx = 1 + blockIdx.x * MUT_TX, by = 1 + blockIdx.y * MUT_TY, bz = 1 + blockIdx.z * MUT_TZ;
+  const T* vel[3] = {W.u, W.v, W.w};
+#pragma unroll 2
+  for (int c = tid; c < RN; c += MUT_TX * MUT_TY) {
+    const int cx = c % RX, r = c / RX, cy = r % RY, cz = r / RY;
+    const int i = bx - 1 + cx, j = by - 1 + cy, k = bz - 1 + cz;
+    if (i < 1 || i > G.nx - 2 || j < 1 || j > G.ny - 2 || k < 1 || k > G.nz - 2) continue;
+    const int64_t o = G.at(i, j, k);
+#pragma unroll
+    for (int q = 0; q < 3; ++q) fv[q * RN + c] = filt(vel[q], o, G.sx, G.plane);
+  }
+  __syncthreads();
+  const int tx = tid % MUT_TX, ty = tid / MUT_TX;
+  const int i = bx + tx, j = by + ty;
+  if (i > G.nx - 2 || j > G.ny - 2) return;
+  const int64_t st[3] = {1, G.sx, G.plane};
+  const int sst[3] = {1, RX, RX * RY};
+  const int n[3] = {G.nx, G.ny, G.nz};
+  const bool per[3] = {!G.bcx, !G.bcy, G.bcz == 0};
+  for (int kk = 0; kk < MUT_TZ; ++kk) {
+    const int k = bz + kk;
+    if (k > G.nz - 2) return;
+    const int64_t o = G.at(i, j, k);
+    const int so = ((kk + 1) * RY + ty + 1) * RX + tx + 1;
+    const T inv[3] = {(T)M.inv_dx[i], (T)M.inv_dy[j], (T)M.inv_dz[k]};
+    const bool inner = mut_inner(G, i, j, k);
+    T a[9], h[9], qc2 = T(0);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        const T* f = vel[c] + o;
+        a[3 * c + d] = T(0.5) * (-f[-st[d]] + f[st[d]]) * inv[d];
+        h[3 * c + d] = a[3 * c + d];
+        if (inner && c != d) {
+          const T* sf = fv + c * RN + so;
+          h[3 * c + d] = T(0.5) * (-sf[-sst[d]] + sf[sst[d]]) * inv[d];
+        }
+      }
+      const T dv = inner ? vel[c][o] - fv[c * RN + so] : T(0);
+      qc2 = c == 0 ? dv * dv : qc2 + dv * dv;
+    }
+    qc2 = T(0.5) * qc2;
+    const T mut = sms_mut<T>(a, h[7] - h[5], h[2] - h[6], h[3] - h[1], qc2, W.rho[o], sms_delta15<T>(G, M, K, i, j, k),
+                             T(K.tan10deg2));
+    W.qc2[o] = qc2;
+    W.mut[o] = mut;
+    // the edge cells this cell is the source of: on each axis at most one (periodic: cell
+    // n-2 serves edge 0 and cell 1 edge n-1; non-periodic: each its own neighbour)
+    const int c3[3] = {i, j, k};
+    int e[3];
+    bool z[3] = {false, false, false}, any = false;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      e[d] = -1;
+      if (c3[d] == 1) e[d] = per[d] ? n[d] - 1 : 0;
+      else if (c3[d] == n[d] - 2) e[d] = per[d] ? 0 : n[d] - 1;
+      if (e[d] < 0) continue;
+      any = true;
+      if (!per[d]) z[d] = ((G.bkind >> (4 * (2 * d + (e[d] ? 1 : 0)))) & 15) == 3;  // no-slip wall: 0
+    }
+    if (!any) continue;
+    for (int m = 1; m < 8; ++m) {
+      int q[3];
+      bool ok = true, zero = false;
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        q[d] = c3[d];
+        if (!((m >> d) & 1)) continue;
+        if (e[d] < 0) ok = false;
+        q[d] = e[d];
+        zero = zero || z[d];
+      }
+      if (!ok) continue;
+      const int64_t p = G.at(q[0], q[1], q[2]);
+      W.mut[p] = zero ? T(0) : mut;
+      W.qc2[p] = zero ? T(0) : qc2;
+    }
+  }
 }
 
 // set_bc_mut_common (3D_solver/src/set_bc_common.f90:296-335): one ghost layer,
@@ -691,14 +763,6 @@ __device__ __forceinline__ void mut_edge_cell(const Geo& G, const Fields<T>& W, 
   const int64_t o = G.at(c[0], c[1], c[2]), src = G.at(s[0], s[1], s[2]);
   W.mut[o] = zero ? T(0) : W.mut[src];
   W.qc2[o] = zero ? T(0) : W.qc2[src];
-}
-
-template <class T>
-__global__ void k_mut_edges(Geo G, Fields<T> W) {
-  int64_t n = (int64_t)G.nx * G.ny * G.nz;
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n;
-       t += (int64_t)gridDim.x * blockDim.x)
-    mut_edge_cell<T>(G, W, t);
 }
 
 // ---- ghost / boundary-cell fill ------------------------------------------------

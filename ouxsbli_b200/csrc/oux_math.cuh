@@ -21,6 +21,7 @@ struct PhysConst {
   double gamma_over_gamma_1, tan10deg2;
   // mixed form only: FP32 pressure / temperature fields hold p - p_ref, T - T_ref
   double p_ref, T_ref;
+  double delta15;  // LES filter width^(3/2) of a grid of uniform spacings (sms_delta15), else 0
 };
 
 template <class T> __device__ __forceinline__ T sgn1(T b) { return signbit(b) ? T(-1) : T(1); }
