@@ -490,7 +490,7 @@ void carve(oux_handle* h) {
 
 // kinds reported by oux_profile_read
 enum KernelKind { KK_PRIM = 0, KK_SENSOR, KK_MUT, KK_MUT_EDGES, KK_SWEEP_X, KK_SWEEP_Y, KK_SWEEP_Z, KK_GHOST,
-                  KK_PRIM_FUSED, KK_GRAD, KK_COUNT };
+                  KK_PRIM_FUSED, KK_GRAD, KK_STAGE2D, KK_COUNT };
 
 struct Timed {
   oux_handle* h;
@@ -651,6 +651,30 @@ int ghost(oux_handle* h, T* Q, cudaStream_t s) {
   return OUX_OK;
 }
 
+// The arguments of stage st of a time step, its combination set:
+// calc_time_dev.f90.fypp:81-101 (RK3), 264-287 (RK4).
+template <class T>
+StepArgs<T> stage_args(oux_handle* h, int st) {
+  StepArgs<T> A = base_args<T>(h);
+  if (h->cfg.rk == 3) {
+    if (st == 0) {
+      A.mode = CM_RK3_1; A.coef = 1.0;
+    } else if (st == 1) {
+      A.mode = CM_RK3_2; A.coef = 0.25; A.c1 = 0.75; A.c2 = 0.25; A.c4 = 1.0;
+    } else {
+      A.mode = CM_RK3_3; A.coef = 2.0; A.c1 = 2.0; A.c2 = 1.0; A.c4 = 1.0 / 3.0;
+    }
+  } else {
+    const double c1[3] = {0.5, 0.5, 1.0}, c2[3] = {1.0, 2.0, 2.0};
+    if (st < 3) {
+      A.mode = CM_RK4_S; A.coef = 1.0; A.c1 = c1[st]; A.c2 = c2[st];
+    } else {
+      A.mode = CM_RK4_4; A.coef = 1.0;
+    }
+  }
+  return A;
+}
+
 // Stage st (0-based) of one time step with compute type T (double: plain FP64 form;
 // float: mixed form), followed by the ghost / boundary fill of the array it wrote.
 template <class T>
@@ -658,27 +682,7 @@ int run_stage_n(oux_handle* h, int st, cudaStream_t s, int part = 0) {
   double* Qn = h->Q;
   T* Qs = reinterpret_cast<T*>(h->Qs);
   const int nst = h->cfg.rk == 3 ? 3 : 4;
-  // the stage's combination: calc_time_dev.f90.fypp:81-101 (RK3), 264-287 (RK4)
-  auto args = [&]() {
-    StepArgs<T> A = base_args<T>(h);
-    if (h->cfg.rk == 3) {
-      if (st == 0) {
-        A.mode = CM_RK3_1; A.coef = 1.0;
-      } else if (st == 1) {
-        A.mode = CM_RK3_2; A.coef = 0.25; A.c1 = 0.75; A.c2 = 0.25; A.c4 = 1.0;
-      } else {
-        A.mode = CM_RK3_3; A.coef = 2.0; A.c1 = 2.0; A.c2 = 1.0; A.c4 = 1.0 / 3.0;
-      }
-    } else {
-      const double c1[3] = {0.5, 0.5, 1.0}, c2[3] = {1.0, 2.0, 2.0};
-      if (st < 3) {
-        A.mode = CM_RK4_S; A.coef = 1.0; A.c1 = c1[st]; A.c2 = c2[st];
-      } else {
-        A.mode = CM_RK4_4; A.coef = 1.0;
-      }
-    }
-    return A;
-  };
+  auto args = [&]() { return stage_args<T>(h, st); };
   // per-cell passes and sweeps over the plane ranges h->G holds
   auto body = [&]() -> int {
     StepArgs<T> A = args();
@@ -736,9 +740,46 @@ int run_stage_n(oux_handle* h, int st, cudaStream_t s, int part = 0) {
   return OUX_OK;
 }
 
+// Whether whole steps of a solve run as one kernel per stage (oux_stage2d.cuh): 2D
+// inviscid, a periodic axis having one cell or at least as many as its ghost cells a side
+// (ghost_cell's image of the others' outer ghost cells is itself a ghost cell).
+bool fused_2d(const oux_handle* h) {
+  const Geo& G = h->G;
+  auto fits = [&](int n, bool wall) { return wall || n == 2 * G.g + 1 || n >= 3 * G.g; };
+  return G.dim == 2 && h->vk == VK_EULER && fits(G.nx, G.bcx) && fits(G.ny, G.bcy);
+}
+
+// nsteps time steps, one kernel per stage.  The stage states alternate between Qs and
+// Racc (no flux differences are stored); in the mixed form Q^n is copied into the field
+// arrays (unused here) by the first stage, and the last one writes the state from there.
+template <class T>
+int run_fused_2d(oux_handle* h, int nsteps, cudaStream_t s) {
+  constexpr bool MX = sizeof(T) < sizeof(double);
+  const int nst = h->cfg.rk == 3 ? 3 : 4;
+  void* const state[2] = {h->Qs, h->Racc};
+  double* const copy = reinterpret_cast<double*>(h->scratch);  // 10 field arrays hold 4 FP64 ones
+  for (int n = 0; n < nsteps; ++n) {
+    for (int st = 0; st < nst; ++st) {
+      StepArgs<T> A = stage_args<T>(h, st);
+      const void* src = st == 0 ? (MX ? nullptr : h->Q) : state[(st - 1) & 1];
+      void* dst = st == nst - 1 ? h->Q : state[st & 1];
+      if (MX && st > 0) A.Qn = copy;
+      int rc;
+      {
+        Timed tm(h, KK_STAGE2D, s);
+        rc = launch_stage2d(h->cfg.order, A, src, dst, MX && st == 0 ? copy : nullptr, s);
+      }
+      if (rc) return fail(OUX_E_CUDA, std::string("2D stage: ") + cudaGetErrorString(cudaGetLastError()));
+      h->launches++;
+    }
+  }
+  return OUX_OK;
+}
+
 // nsteps time steps
 template <class T>
 int run_steps(oux_handle* h, int nsteps, cudaStream_t s) {
+  if (fused_2d(h)) return run_fused_2d<T>(h, nsteps, s);
   const int nst = h->cfg.rk == 3 ? 3 : 4;
   for (int n = 0; n < nsteps; ++n)
     for (int st = 0; st < nst; ++st) {

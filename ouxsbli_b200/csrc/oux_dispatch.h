@@ -39,4 +39,14 @@ inline int launch_sweep_dir_mx(int dim, int order, int vk, bool les, int dir, co
 inline int launch_sweeps_mx(int dim, int order, int vk, bool les, const StepArgs<float>& A, cudaStream_t s) {
   return launch_sweep_dir_mx(dim, order, vk, les, -1, A, s);
 }
+
+// one stage of a 2D inviscid solve (oux_stage2d.cuh)
+int launch_stage2d_fp64(int order, const StepArgs<double>& A, const void* src, void* dst, double* keep, cudaStream_t s);
+int launch_stage2d_mx(int order, const StepArgs<float>& A, const void* src, void* dst, double* keep, cudaStream_t s);
+inline int launch_stage2d(int order, const StepArgs<double>& A, const void* src, void* dst, double* keep, cudaStream_t s) {
+  return launch_stage2d_fp64(order, A, src, dst, keep, s);
+}
+inline int launch_stage2d(int order, const StepArgs<float>& A, const void* src, void* dst, double* keep, cudaStream_t s) {
+  return launch_stage2d_mx(order, A, src, dst, keep, s);
+}
 }  // namespace oux

@@ -137,20 +137,28 @@ inline dim3 plane_grid(const Geo& G) {
 }
 
 // ---- prim: src/calc_physical_quantities.f90:60-116 (3D), :7-57 (2D) -------
+// Density, velocities, pressure and temperature of a cell from its FP64 conservative values q.
+template <int DIM>
+__device__ __forceinline__ void prim_decode(const double* q, double Jv, const PhysConst& K, double& rho,
+                                            double (&v)[3], double& p, double& temp) {
+  const double over = 1.0 / q[0];
+  rho = Jv * q[0];
+  v[0] = q[1] * over;
+  v[1] = q[2] * over;
+  v[2] = DIM == 3 ? q[3] * over : 0.0;
+  if constexpr (DIM == 3) p = K.gamma_1 * (Jv * q[4] - 0.5 * rho * (v[0] * v[0] + v[1] * v[1] + v[2] * v[2]));
+  else p = K.gamma_1 * (Jv * q[3] - 0.5 * rho * (v[0] * v[0] + v[1] * v[1]));
+  temp = p / (K.R * rho);
+}
+
 // The primitive fields of a cell from its FP64 conservative values q (mixed form MX: p
 // and T stored as deviations from K.p_ref, K.T_ref, everything rounded once); v returns
 // the velocities in FP64.
 template <int DIM, bool VISC, bool MX, class T>
 __device__ __forceinline__ void prim_store(const double* q, double Jv, const Fields<T>& W, int64_t o,
                                            const PhysConst& K, double (&v)[3]) {
-  const double over = 1.0 / q[0], rho = Jv * q[0];
-  v[0] = q[1] * over;
-  v[1] = q[2] * over;
-  v[2] = DIM == 3 ? q[3] * over : 0.0;
-  double p;
-  if constexpr (DIM == 3) p = K.gamma_1 * (Jv * q[4] - 0.5 * rho * (v[0] * v[0] + v[1] * v[1] + v[2] * v[2]));
-  else p = K.gamma_1 * (Jv * q[3] - 0.5 * rho * (v[0] * v[0] + v[1] * v[1]));
-  const double temp = p / (K.R * rho);
+  double rho, p, temp;
+  prim_decode<DIM>(q, Jv, K, rho, v, p, temp);
   W.rho[o] = (T)rho;
   W.u[o] = (T)v[0];
   W.v[o] = (T)v[1];
@@ -225,16 +233,22 @@ __global__ void __launch_bounds__(PLANE_THREADS) k_prim_mx(const double* __restr
 // vel_c(o + st_a) of velocity component c along axis a (the caller has checked that
 // the cell lies in 1..n-2 on every axis), so that a pass which has loaded those
 // neighbours already (k_grad) reuses them.
-// The sensor value from the summed divergence and the rotation components, stored
-// with the reference's copies to the outer faces (3D: r1, r2, r3; 2D: r3 = rot).
+// The sensor value from the summed divergence and the rotation components (3D: r1, r2,
+// r3; 2D: r3 = rot).
 template <int DIM, class T>
-__device__ __forceinline__ void ducros_store(const Geo& G, const Fields<T>& W, int i, int j, int k, T div, T r1,
-                                             T r2, T r3) {
+__device__ __forceinline__ T ducros_value(T div, T r1, T r2, T r3) {
   const T eps = T(1.0e-12);
   T f;
   if constexpr (DIM == 3) f = (div * div) / (div * div + (r1 * r1 + r2 * r2 + r3 * r3) + eps);
   else f = (div * div) / (div * div + r3 * r3 + eps);
-  f = fmin_f(T(1), f);
+  return fmin_f(T(1), f);
+}
+
+// ... stored with the reference's copies to the outer faces.
+template <int DIM, class T>
+__device__ __forceinline__ void ducros_store(const Geo& G, const Fields<T>& W, int i, int j, int k, T div, T r1,
+                                             T r2, T r3) {
+  const T f = ducros_value<DIM, T>(div, r1, r2, r3);
   W.sensor[G.at(i, j, k)] = f;
   if (i == 1) W.sensor[G.at(0, j, k)] = f; else if (i == G.nx - 2) W.sensor[G.at(G.nx - 1, j, k)] = f;
   if (j == 1) W.sensor[G.at(i, 0, k)] = f; else if (j == G.ny - 2) W.sensor[G.at(i, G.ny - 1, k)] = f;
@@ -950,6 +964,28 @@ __device__ __forceinline__ void ghost_cell_3d_bnd(T* Q, const Geo& G, int nv, in
   }
 }
 
+// The value of boundary cell (i, j) of a 2D grid from that of its source cell (si, sj),
+// in place.  A corner takes the rule applied last, to the other direction's boundary
+// value beside it.
+__device__ __forceinline__ void bc_2d(const Geo& G, int nv, double (&v)[5], int i, int j, int si, int sj) {
+  const bool xb = G.bcx && (i == 0 || i == G.nx - 1), yb = G.bcy && (j == 0 || j == G.ny - 1);
+  const int fx = i == 0 ? 0 : 1, fy = j == 0 ? 2 : 3;
+  const int64_t nx = G.nx;
+  if (xb && yb) {
+    if (!G.ylast) {
+      bc_rule(G, fy, si, nv, v, j * nx + si, sj * nx + si);
+      bc_rule(G, fx, j, nv, v, j * nx + i, j * nx + si);
+    } else {
+      bc_rule(G, fx, sj, nv, v, sj * nx + i, sj * nx + si);
+      bc_rule(G, fy, i, nv, v, j * nx + i, sj * nx + i);
+    }
+  } else if (xb) {
+    bc_rule(G, fx, j, nv, v, sj * nx + i, sj * nx + si);
+  } else if (yb) {
+    bc_rule(G, fy, i, nv, v, j * nx + si, sj * nx + si);
+  }
+}
+
 // Qn: null for a full state Q; in the mixed form Q holds FP32 stage increments over
 // the FP64 state Qn, and a boundary rule is applied to Qn + Q (the increment stored
 // is the rule's state minus Qn), so it acts as on a full state.
@@ -990,41 +1026,17 @@ __device__ __forceinline__ void ghost_cell(T* Q, const Geo& G, int nv, int64_t t
     for (int l = 0; l < nv; ++l) Q[o + l * G.vs] = Q[s + l * G.vs];
     return;
   }
-  double v[5];
-  auto load = [&](int64_t s) {
-    for (int l = 0; l < nv; ++l) {
-      const int64_t q = s + l * G.vs;
-      v[l] = Qn ? Qn[q] + (double)Q[q] : (double)Q[q];
-    }
-  };
+  // the source cell: the neighbour across a boundary, the image along a periodic axis
+  const int si = !G.bcx ? (i - gx + Nx) % Nx + gx : i == 0 ? 1 : i == G.nx - 1 ? G.nx - 2 : i;
+  const int sj = !G.bcy ? (j - gy + Ny) % Ny + gy : j == 0 ? 1 : j == G.ny - 1 ? G.ny - 2 : j;
   const int sk = (G.dim == 3) ? (k - g + Nz) % Nz + g : 0;
-  const int64_t nx = G.nx;
-  if (xb && yb) {
-    // corner: the rule applied last, to the other direction's boundary value beside it
-    const int fx = i == 0 ? 0 : 1, in = i == 0 ? 1 : G.nx - 2;
-    const int fy = j == 0 ? 2 : 3, jn = j == 0 ? 1 : G.ny - 2;
-    load(G.at(in, jn, sk));
-    if (!G.ylast) {
-      bc_rule(G, fy, in, nv, v, j * nx + in, jn * nx + in);
-      bc_rule(G, fx, j, nv, v, j * nx + i, j * nx + in);
-    } else {
-      bc_rule(G, fx, jn, nv, v, jn * nx + i, jn * nx + in);
-      bc_rule(G, fy, i, nv, v, j * nx + i, jn * nx + i);
-    }
-  } else if (xb) {
-    // x face: the neighbour column's value in this row (a periodic image of an
-    // interior row when y is periodic)
-    const int fx = i == 0 ? 0 : 1, in = i == 0 ? 1 : G.nx - 2;
-    const int sj = G.bcy ? j : (j - gy + Ny) % Ny + gy;
-    load(G.at(in, sj, sk));
-    bc_rule(G, fx, j, nv, v, sj * nx + i, sj * nx + in);
-  } else {
-    // y face of an interior column (or a periodic-x ghost column's image)
-    const int fy = j == 0 ? 2 : 3, jn = j == 0 ? 1 : G.ny - 2;
-    const int si = G.bcx ? i : (i - gx + Nx) % Nx + gx;
-    load(G.at(si, jn, sk));
-    bc_rule(G, fy, i, nv, v, j * nx + si, jn * nx + si);
+  const int64_t s = G.at(si, sj, sk);
+  double v[5];
+  for (int l = 0; l < nv; ++l) {
+    const int64_t q = s + l * G.vs;
+    v[l] = Qn ? Qn[q] + (double)Q[q] : (double)Q[q];
   }
+  bc_2d(G, nv, v, i, j, si, sj);
   for (int l = 0; l < nv; ++l) {
     const int64_t q = o + l * G.vs;
     Q[q] = Qn ? (T)(v[l] - Qn[q]) : (T)v[l];

@@ -764,6 +764,176 @@ namespace oux {
 #ifndef OUX_SWEEP_MINB_YZ
 #define OUX_SWEEP_MINB_YZ 2
 #endif
+// Flux of the face whose left cell is fc (padded indices): the convective flux and,
+// unless the caller combines shared ME4 positions itself (SHARE), minus the viscous one.
+// st0(field, m) reads the tile field of cell f - 2 + m along DIR, m = 0 .. 5.
+template <int DIM, int DIR, int ORDER, int VK, bool LES, class T, bool RO, bool KONLY, bool SHARE, class Acc>
+__device__ __forceinline__ void face_flux(const StepArgs<T>& A, const Acc& st0, const int fc[3], T F[5]) {
+  constexpr int H = ORDER / 2;
+  constexpr int VB = vk_base(VK);
+  constexpr bool WALL = vk_wall(VK);
+  const Geo& G = A.G;
+  const int f = fc[DIR];
+  const int64_t stv[3] = {1, G.sx, G.plane};
+  auto sc = [&](int field, int m) -> T { return st0(field, m + TILE_HALO - H); };
+  T fd = T(0);
+  if (!KONLY && A.scheme != 0) fd = T(0.5) * (st0(TF_SEN, 2) + st0(TF_SEN, 3));
+  if constexpr (DIM == 2 || VK == VK_EULER || WALL) {
+    // non-periodic x / y (/ z): every face, the stencil order lowered next to the
+    // boundary as the reference's boundary kernels do (2D_solver/src/calc_{slau,
+    // keep,hybrid}_kernel.f90.fypp, calc_*_x and calc_*_y; 3D_solver/src/calc_*
+    // _kernel.f90.fypp): 6th for 2 <= f <= n-4, 4th for 1 <= f <= n-3, else 2nd /
+    // first order (f: 0-based left cell of the face).  Compiled out of the periodic
+    // 3D viscous sweeps (their walled variants carry it).
+    int lo = ORDER;
+    const int nn = DIR == 0 ? G.nx : (DIR == 1 ? G.ny : G.nz);
+    const bool nonper = DIR == 0 ? (bool)G.bcx : (DIR == 1 ? (bool)G.bcy : G.bcz == 1);
+    if (nonper)
+      lo = (ORDER == 6 && f >= 2 && f <= nn - 4) ? 6 : (ORDER >= 4 && f >= 1 && f <= nn - 3) ? 4 : 2;
+    if (lo == ORDER) {
+      conv_flux<ORDER, KONLY>(A, sc, fd, DIR, F);
+    } else if (lo == 4) {
+      auto s4 = [&](int field, int m) -> T { return st0(field, m + TILE_HALO - 2); };
+      conv_flux<4, KONLY>(A, s4, fd, DIR, F);
+    } else {
+      auto s2 = [&](int field, int m) -> T { return st0(field, m + TILE_HALO - 1); };
+      conv_flux<2, KONLY>(A, s2, fd, DIR, F);
+    }
+  } else {
+    conv_flux<ORDER, KONLY>(A, sc, fd, DIR, F);
+  }
+  if constexpr (VK != VK_EULER && !SHARE) {
+    T vo[4];
+    const double* invd[3] = {A.M.inv_dx, A.M.inv_dy, A.M.inv_dz};
+    const T inv = (T)invd[DIR][f];
+    if constexpr (VB == VK_GV2) {
+      const int64_t o = G.at(fc[0], fc[1], DIM == 3 ? fc[2] : 0);
+      T invs[3] = {(T)A.M.inv_dx[fc[0]], (T)A.M.inv_dy[fc[1]], DIM == 3 ? (T)A.M.inv_dz[fc[2]] : T(0)};
+      visc_gv2<DIM, LES, RO>(A, DIR, o, stv, invs, vo);
+    } else if constexpr (VK == VK_2D4) {
+      // inner guard of calc_Ev4 / calc_Fv4 (2D): face 2..n-4, transverse 2..n-3
+      const int nt = DIR == 0 ? G.ny : G.nx;
+      const int tr = fc[1 - DIR];
+      const int nn = DIR == 0 ? G.nx : G.ny;
+      bool inner = (f >= 2 && f <= nn - 4 && tr >= 2 && tr <= nt - 3);
+      const int64_t o = G.at(fc[0], fc[1], 0);
+      T invs[2] = {(T)A.M.inv_dx[fc[0]], (T)A.M.inv_dy[fc[1]]};
+      invs[DIR] = inv;
+      visc_2d4(A, st0, DIR, inner, o, stv, invs, vo);
+    } else {
+      constexpr int off0 = (VB == VK_C4) ? -1 : -2;
+      auto sv = [&](int field, int m) -> T { return st0(field, m + 2 + off0); };
+      if constexpr (WALL) {
+        // high-order guard of calc_{E,F,G}v (calc_visc_high.f90.fypp:114/139/169,
+        // 350/376/406, 592/618/648), 0-based: C4 faces 1..n-3 and transverse cells
+        // 2..n-3, ME4 faces 2..n-4 and cells 2..n-3, C6 faces 2..n-4 and cells 3..n-4
+        constexpr int FA = (VB == VK_C4) ? 1 : 2, TA = (VB == VK_C6) ? 3 : 2;
+        const int na[3] = {G.nx, G.ny, G.nz};
+        bool inner = f >= FA && f <= na[DIR] - 2 - FA;
+#pragma unroll
+        for (int a = 0; a < 3; ++a)
+          if (a != DIR) inner = inner && fc[a] >= TA && fc[a] <= na[a] - 1 - TA;
+        if (inner) {
+          visc_high<VB, LES>(A, sv, DIR, inv, vo);
+        } else {
+          const int64_t o = G.at(fc[0], fc[1], fc[2]);
+          T invs[3] = {(T)A.M.inv_dx[fc[0]], (T)A.M.inv_dy[fc[1]], (T)A.M.inv_dz[fc[2]]};
+          invs[DIR] = inv;
+          visc_fb3<LES>(A, DIR, o, stv, invs, vo);
+        }
+      } else {
+        visc_high<VB, LES>(A, sv, DIR, inv, vo);
+      }
+    }
+    if constexpr (DIM == 3) {
+      F[1] = F[1] - vo[0]; F[2] = F[2] - vo[1]; F[3] = F[3] - vo[2]; F[4] = F[4] - vo[3];
+    } else {
+      F[1] = F[1] - vo[0]; F[2] = F[2] - vo[1]; F[4] = F[4] - vo[3];
+    }
+  }
+}
+
+// dt * S metric of a cell's faces along DIR (calc_steps.f90 calc_R).
+template <int DIM, int DIR, class T>
+__device__ __forceinline__ double face_metric(const StepArgs<T>& A, int i, int j, int k) {
+  const Geo& G = A.G;
+  if constexpr (DIM == 3) {
+    if (DIR == 0) return A.M.dtdydz[(int64_t)(k - 1) * (G.ny - 2) + (j - 1)];
+    if (DIR == 1) return A.M.dtdzdx[(int64_t)(k - 1) * (G.nx - 2) + (i - 1)];
+    return A.M.dtdxdy[(int64_t)(j - 1) * (G.nx - 2) + (i - 1)];
+  } else {
+    return (DIR == 0) ? A.M.dtdy[j - 1] : A.M.dtdx[i - 1];
+  }
+}
+
+// The stage's Runge-Kutta combination of cell (i, j, k), offset o, from its residual R
+// (or the residual itself, CM_R_OUT); QN, QS, RS read the operands.
+template <int DIM, class T, class FQN, class FQS, class FRS>
+__device__ __forceinline__ void combine_cell(const StepArgs<T>& A, int i, int j, int k, int64_t o,
+                                             const double (&R)[DIM + 2], FQN QN, FQS QS, FRS RS) {
+  constexpr int NV = DIM + 2;
+  constexpr bool MXC = sizeof(T) < sizeof(double);
+  const Geo& G = A.G;
+  // mixed form: the stage state holds the FP32 increment Q^(s) - Q^n
+  switch (A.mode) {
+    case CM_R_OUT: {
+      // reference Rs(nx-2, nv, ny-2, nz-2) order, cell (i,j,k) -> (i-1, l, j-1, k-1)
+      int64_t base = (((int64_t)(DIM == 3 ? k - 1 : 0) * (G.ny - 2) + (j - 1)) * NV) * (G.nx - 2) + (i - 1);
+#pragma unroll
+      for (int l = 0; l < NV; ++l) A.Rout[base + (int64_t)l * (G.nx - 2)] = R[l];
+      break;
+    }
+    case CM_RK3_1: {
+#pragma unroll
+      for (int l = 0; l < NV; ++l) {
+        const int64_t q = o + l * G.vs;
+        if constexpr (MXC) A.Qs[q] = (T)(-R[l]);  // stage increment Q1 - Qn
+        else A.Qs[q] = (T)(QN(l) - R[l]);
+      }
+      break;
+    }
+    case CM_RK3_2: {
+#pragma unroll
+      for (int l = 0; l < NV; ++l) {
+        const int64_t q = o + l * G.vs;
+        if constexpr (MXC) A.Qs[q] = (T)((A.c2 * (double)QS(l) - R[l]) * A.c4);  // c1 + c2 = 1
+        else A.Qs[q] = (T)((A.c1 * QN(l) + A.c2 * (double)QS(l) - R[l]) * A.c4);
+      }
+      break;
+    }
+    case CM_RK3_3: {
+#pragma unroll
+      for (int l = 0; l < NV; ++l) {
+        const int64_t q = o + l * G.vs;
+        if constexpr (MXC) A.Qn[q] = QN(l) + (A.c1 * (double)QS(l) - R[l]) * A.c4;  // (c1 + c2) c4 = 1
+        else A.Qn[q] = (A.c1 * (double)QS(l) + A.c2 * QN(l) - R[l]) * A.c4;
+      }
+      break;
+    }
+    case CM_RK4_S: {
+#pragma unroll
+      for (int l = 0; l < NV; ++l) {
+        const int64_t q = o + l * G.vs;
+        if constexpr (MXC) A.Qs[q] = (T)(-A.c1 * R[l]);
+        else A.Qs[q] = (T)(QN(l) - A.c1 * R[l]);
+        A.Rs[q] = RS(l) + A.c2 * R[l];
+      }
+      break;
+    }
+    case CM_RK4_4: {
+#pragma unroll
+      for (int l = 0; l < NV; ++l) {
+        const int64_t q = o + l * G.vs;
+        double r = RS(l) + R[l];
+        A.Qn[q] = QN(l) - r * (1.0 / 6.0);
+        A.Rs[q] = 0.0;
+      }
+      break;
+    }
+    default: break;
+  }
+}
+
 // One sweep tile: block-tile indices (b0, b1, b2) as the grid of launch_one
 // enumerates them; `tid` / `nthr_all` are the calling block's linear thread index
 // and size (>= TX*TY: threads beyond the tile shape only help load the tile).
@@ -1072,85 +1242,7 @@ __device__ __forceinline__ void sweep_tile(const StepArgs<T>& A, int last, int b
       T F[5];
       // tile position of cell f + off is base + (2 + off) * step
       auto st0 = [&](int field, int m) -> T { return tile[field * FS + base + m * step]; };
-      const int cb = base + (TILE_HALO - H) * step;
-      auto sc = [&](int field, int m) -> T { return tile[field * FS + cb + m * step]; };
-      T fd = T(0);
-      if (!KONLY && A.scheme != 0) fd = T(0.5) * (st0(TF_SEN, 2) + st0(TF_SEN, 3));
-      if constexpr (DIM == 2 || VK == VK_EULER || WALL) {
-        // non-periodic x / y (/ z): every face, the stencil order lowered next to the
-        // boundary as the reference's boundary kernels do (2D_solver/src/calc_{slau,
-        // keep,hybrid}_kernel.f90.fypp, calc_*_x and calc_*_y; 3D_solver/src/calc_*
-        // _kernel.f90.fypp): 6th for 2 <= f <= n-4, 4th for 1 <= f <= n-3, else 2nd /
-        // first order (f: 0-based left cell of the face).  Compiled out of the periodic
-        // 3D viscous sweeps (their walled variants carry it).
-        int lo = ORDER;
-        const int nn = DIR == 0 ? G.nx : (DIR == 1 ? G.ny : G.nz);
-        const bool nonper = DIR == 0 ? (bool)G.bcx : (DIR == 1 ? (bool)G.bcy : G.bcz == 1);
-        if (nonper)
-          lo = (ORDER == 6 && f >= 2 && f <= nn - 4) ? 6 : (ORDER >= 4 && f >= 1 && f <= nn - 3) ? 4 : 2;
-        if (lo == ORDER) {
-          conv_flux<ORDER, KONLY>(A, sc, fd, DIR, F);
-        } else if (lo == 4) {
-          auto s4 = [&](int field, int m) -> T { return tile[field * FS + base + (TILE_HALO - 2 + m) * step]; };
-          conv_flux<4, KONLY>(A, s4, fd, DIR, F);
-        } else {
-          auto s2 = [&](int field, int m) -> T { return tile[field * FS + base + (TILE_HALO - 1 + m) * step]; };
-          conv_flux<2, KONLY>(A, s2, fd, DIR, F);
-        }
-      } else {
-        conv_flux<ORDER, KONLY>(A, sc, fd, DIR, F);
-      }
-      if constexpr (VK != VK_EULER && !SHARE) {
-        T vo[4];
-        const double* invd[3] = {A.M.inv_dx, A.M.inv_dy, A.M.inv_dz};
-        const T inv = (T)invd[DIR][f];
-        if constexpr (VB == VK_GV2) {
-          const int64_t o = G.at(fc[0], fc[1], DIM == 3 ? fc[2] : 0);
-          T invs[3] = {(T)A.M.inv_dx[fc[0]], (T)A.M.inv_dy[fc[1]], DIM == 3 ? (T)A.M.inv_dz[fc[2]] : T(0)};
-          visc_gv2<DIM, LES, RO>(A, DIR, o, stv, invs, vo);
-        } else if constexpr (VK == VK_2D4) {
-          // inner guard of calc_Ev4 / calc_Fv4 (2D): face 2..n-4, transverse 2..n-3
-          const int nt = DIR == 0 ? G.ny : G.nx;
-          const int tr = fc[1 - DIR];
-          const int nn = DIR == 0 ? G.nx : G.ny;
-          bool inner = (f >= 2 && f <= nn - 4 && tr >= 2 && tr <= nt - 3);
-          const int64_t o = G.at(fc[0], fc[1], 0);
-          T invs[2] = {(T)A.M.inv_dx[fc[0]], (T)A.M.inv_dy[fc[1]]};
-          invs[DIR] = inv;
-          auto sv = [&](int field, int m) -> T { return tile[field * FS + base + m * step]; };
-          visc_2d4(A, sv, DIR, inner, o, stv, invs, vo);
-        } else {
-          constexpr int off0 = (VB == VK_C4) ? -1 : -2;
-          const int vb = base + (2 + off0) * step;
-          auto sv = [&](int field, int m) -> T { return tile[field * FS + vb + m * step]; };
-          if constexpr (WALL) {
-            // high-order guard of calc_{E,F,G}v (calc_visc_high.f90.fypp:114/139/169,
-            // 350/376/406, 592/618/648), 0-based: C4 faces 1..n-3 and transverse cells
-            // 2..n-3, ME4 faces 2..n-4 and cells 2..n-3, C6 faces 2..n-4 and cells 3..n-4
-            constexpr int FA = (VB == VK_C4) ? 1 : 2, TA = (VB == VK_C6) ? 3 : 2;
-            const int na[3] = {G.nx, G.ny, G.nz};
-            bool inner = f >= FA && f <= na[DIR] - 2 - FA;
-#pragma unroll
-            for (int a = 0; a < 3; ++a)
-              if (a != DIR) inner = inner && fc[a] >= TA && fc[a] <= na[a] - 1 - TA;
-            if (inner) {
-              visc_high<VB, LES>(A, sv, DIR, inv, vo);
-            } else {
-              const int64_t o = G.at(fc[0], fc[1], fc[2]);
-              T invs[3] = {(T)A.M.inv_dx[fc[0]], (T)A.M.inv_dy[fc[1]], (T)A.M.inv_dz[fc[2]]};
-              invs[DIR] = inv;
-              visc_fb3<LES>(A, DIR, o, stv, invs, vo);
-            }
-          } else {
-            visc_high<VB, LES>(A, sv, DIR, inv, vo);
-          }
-        }
-        if constexpr (DIM == 3) {
-          F[1] = F[1] - vo[0]; F[2] = F[2] - vo[1]; F[3] = F[3] - vo[2]; F[4] = F[4] - vo[3];
-        } else {
-          F[1] = F[1] - vo[0]; F[2] = F[2] - vo[1]; F[4] = F[4] - vo[3];
-        }
-      }
+      face_flux<DIM, DIR, ORDER, VK, LES, T, RO, KONLY, SHARE>(A, st0, fc, F);
 #pragma unroll
       for (int l = 0; l < 5; ++l) Fs[l * (TX * TY) + tid] = (double)F[l];
     }
@@ -1213,16 +1305,7 @@ __device__ __forceinline__ void sweep_tile(const StepArgs<T>& A, int last, int b
       if constexpr (PF_C) return pfRs[l * PFC + slot];
       else return A.Rs[o + l * G.vs];
     };
-    // dt * S metric for this direction, scaled by coef (calc_steps.f90 calc_R)
-    double met;
-    if constexpr (DIM == 3) {
-      if (DIR == 0) met = A.M.dtdydz[(int64_t)(k - 1) * (G.ny - 2) + (j - 1)];
-      else if (DIR == 1) met = A.M.dtdzdx[(int64_t)(k - 1) * (G.nx - 2) + (i - 1)];
-      else met = A.M.dtdxdy[(int64_t)(j - 1) * (G.nx - 2) + (i - 1)];
-    } else {
-      met = (DIR == 0) ? A.M.dtdy[j - 1] : A.M.dtdx[i - 1];
-    }
-    const double cm = A.coef * met;
+    const double cm = A.coef * face_metric<DIM, DIR>(A, i, j, k);
     constexpr int NV = DIM + 2;
     double R[NV];
 #pragma unroll
@@ -1237,64 +1320,7 @@ __device__ __forceinline__ void sweep_tile(const StepArgs<T>& A, int last, int b
       for (int l = 0; l < NV; ++l) A.Racc[o + l * G.vs] = R[l];
       return;
     }
-    // mixed form: the stage state holds the FP32 increment Q^(s) - Q^n
-    switch (A.mode) {
-      case CM_R_OUT: {
-        // reference Rs(nx-2, nv, ny-2, nz-2) order, cell (i,j,k) -> (i-1, l, j-1, k-1)
-        int64_t base = (((int64_t)(DIM == 3 ? k - 1 : 0) * (G.ny - 2) + (j - 1)) * NV) * (G.nx - 2) + (i - 1);
-#pragma unroll
-        for (int l = 0; l < NV; ++l) A.Rout[base + (int64_t)l * (G.nx - 2)] = R[l];
-        break;
-      }
-      case CM_RK3_1: {
-#pragma unroll
-        for (int l = 0; l < NV; ++l) {
-          const int64_t q = o + l * G.vs;
-          if constexpr (MXC) A.Qs[q] = (T)(-R[l]);  // stage increment Q1 - Qn
-          else A.Qs[q] = (T)(QN(l) - R[l]);
-        }
-        break;
-      }
-      case CM_RK3_2: {
-#pragma unroll
-        for (int l = 0; l < NV; ++l) {
-          const int64_t q = o + l * G.vs;
-          if constexpr (MXC) A.Qs[q] = (T)((A.c2 * (double)QS(l) - R[l]) * A.c4);  // c1 + c2 = 1
-          else A.Qs[q] = (T)((A.c1 * QN(l) + A.c2 * (double)QS(l) - R[l]) * A.c4);
-        }
-        break;
-      }
-      case CM_RK3_3: {
-#pragma unroll
-        for (int l = 0; l < NV; ++l) {
-          const int64_t q = o + l * G.vs;
-          if constexpr (MXC) A.Qn[q] = QN(l) + (A.c1 * (double)QS(l) - R[l]) * A.c4;  // (c1 + c2) c4 = 1
-          else A.Qn[q] = (A.c1 * (double)QS(l) + A.c2 * QN(l) - R[l]) * A.c4;
-        }
-        break;
-      }
-      case CM_RK4_S: {
-#pragma unroll
-        for (int l = 0; l < NV; ++l) {
-          const int64_t q = o + l * G.vs;
-          if constexpr (MXC) A.Qs[q] = (T)(-A.c1 * R[l]);
-          else A.Qs[q] = (T)(QN(l) - A.c1 * R[l]);
-          A.Rs[q] = RS(l) + A.c2 * R[l];
-        }
-        break;
-      }
-      case CM_RK4_4: {
-#pragma unroll
-        for (int l = 0; l < NV; ++l) {
-          const int64_t q = o + l * G.vs;
-          double r = RS(l) + R[l];
-          A.Qn[q] = QN(l) - r * (1.0 / 6.0);
-          A.Rs[q] = 0.0;
-        }
-        break;
-      }
-      default: break;
-    }
+    combine_cell<DIM>(A, i, j, k, o, R, QN, QS, RS);
   }
 }
 
