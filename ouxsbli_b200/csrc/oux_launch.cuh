@@ -1,12 +1,26 @@
 // Grid/block/shared-memory setup for the three sweeps of one stage.
 #pragma once
 #include <cstring>
+#include "oux_march.cuh"
 #include "oux_sweep.cuh"
 
 namespace oux {
 
 template <int DIM, int DIR, int ORDER, int VK, bool LES, class T, bool SHARE = false>
 int launch_one(const StepArgs<T>& A, int last, cudaStream_t s) {
+  if constexpr (DIM == 3 && sweep_uses_grads<DIM, VK>() && !SHARE) {
+    // marching sweeps from the size on where they are the faster ones (march_min_cells)
+    const int64_t cells = (int64_t)(A.G.nx - 2 * A.G.gx) * (A.G.ny - 2 * A.G.gy) * (A.G.sk1 - A.G.sk0);
+    const bool share = VK == VK_ME4 && ((A.G.uni >> DIR) & 1);
+    if constexpr (VK == VK_ME4) {
+      if (share && cells >= march_min_cells<DIR, T, true>())
+        return launch_march_dir<DIR, ORDER, VK, LES, T, true>(A, s);
+    }
+    if constexpr (march_min_cells<DIR, T, false>() != INT64_MAX) {
+      if (!share && cells >= march_min_cells<DIR, T, false>())
+        return launch_march_dir<DIR, ORDER, VK, LES, T, false>(A, s);
+    }
+  }
   // ME4 on an axis of uniform spacing: the shared-position variant of the x and y
   // sweeps (measured on B200 at 512^3: y 9.98 -> 9.66 ms, x unchanged; the z sweep,
   // whose operand prefetch already holds 82 KB of shared memory per block, lost L1

@@ -170,3 +170,79 @@ def test_fused_2d_mixed(n, bc, scheme, rk):
     a, b = s.get_state(), oracle.step(cfg, qj, 3)
     for l in range(4):
         assert np.abs(a[:, l] - b[:, l]).max() <= 2e-6 * np.abs(b).max()
+
+
+# ---- marching sweeps (oux_march.cuh): from 380 000 interior cells (FP64; x and y), 6 000 000 (z, ME4), mixed 100 000 and 11 000 000 ----
+# extents one past, at and short of 32 columns (x, z) and of 8 (y), segments of one row and of
+# odd lengths, axes of 1 to 3 cells, rows longer than a warp's ring
+XY_SIZES = [(33, 109, 107), (31, 113, 110), (512, 28, 27), (95, 3, 1340), (3, 350, 366), (620, 613, 1)]
+Z_SIZES = [(97, 251, 249), (33, 430, 426), (1, 2457, 2443)]
+
+
+@pytest.mark.parametrize("n", XY_SIZES + Z_SIZES)
+def test_marching_sweeps_me4(n):
+    cfg, qj = box(n, scheme="Hybrid", visc="NS", visc_stencil="ME4Base")
+    a, b = residuals(cfg, qj)
+    assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("kw", [
+    dict(scheme="SLAU", visc="NS"), dict(scheme="KEEP", visc="NS", rk=4), dict(scheme="Roe", visc="NS", visc_order=4),
+    dict(scheme="Hybrid", visc="NS", visc_stencil="ME4Base", stretch=True),
+    dict(order=4, scheme="Hybrid", visc="NS", visc_order=4)])
+@pytest.mark.parametrize("n", [(65, 77, 79), (97, 113, 111)])
+def test_marching_sweeps_stencils(n, kw):
+    cfg, qj = box(n, **kw)
+    a, b = residuals(cfg, qj)
+    assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("rk", [3, 4])
+@pytest.mark.parametrize("n", [(65, 77, 79), (182, 184, 183)])
+def test_marching_sweeps_stage_combinations(n, rk):
+    """Whole steps: the z sweep's combinations of RK3 and RK4 with their operands."""
+    from ouxsbli_b200.solver import Solver
+    cfg, qj = box(n, scheme="Hybrid", visc="NS", visc_stencil="ME4Base", rk=rk)
+    s = Solver(cfg)
+    s.set_state(qj)
+    s.step(1)
+    assert np.array_equal(s.get_state(), oracle.step(cfg, qj, 1))
+
+
+@pytest.mark.parametrize("stencil", ["Central", "ME4Base"])
+@pytest.mark.parametrize("n", [(65, 77, 79), (97, 113, 111)])
+def test_marching_sweeps_les(n, stencil):
+    cfg, qj = box(n, scheme="SLAU", visc="LES", visc_stencil=stencil)
+    a, b = residuals(cfg, qj)
+    assert np.abs(a - b).max() <= 1e-11 * np.abs(b).max()
+
+
+@pytest.mark.parametrize("n,rk", [((65, 77, 79), 3), ((65, 77, 79), 4), ((225, 223, 221), 3)])
+def test_marching_sweeps_mixed(n, rk):
+    """One mixed step: increments rounded to FP32 and FP32 fluxes of smooth fields, as above."""
+    from ouxsbli_b200.solver import Solver
+    cfg, qj = box(n, scheme="KEEP", visc="NS", visc_stencil="ME4Base", rk=rk, precision="mixed")
+    s = Solver(cfg)
+    s.set_state(qj)
+    s.step(1)
+    a, b = s.get_state(), oracle.step(cfg, qj, 1)
+    for l in range(5):
+        assert np.abs(a[:, l] - b[:, l]).max() <= 2e-6 * np.abs(b[:, 1:4] if 1 <= l <= 3 else b[:, l]).max()
+
+
+@pytest.mark.parametrize("stencil,visc", [("Central", "NS"), ("ME4Base", "NS"), ("Central", "LES")])
+def test_marching_sweeps_walls(stencil, visc):
+    """Walls on every axis: the order fallback and the 2nd-order viscous faces."""
+    from helpers import wall_box
+    rules = {"x_lo": "slip_wall", "x_hi": "slip_wall", "y_lo": "noslip_wall", "y_hi": "noslip_wall",
+             "z_lo": "slip_wall", "z_hi": "noslip_wall"}
+    cfg, qj, _ = wall_box(97, 115, 111, 6, rules, bc_x=1, bc_z=1, scheme="Hybrid", visc=visc, visc_stencil=stencil)
+    from ouxsbli_b200.solver import Solver
+    qj = oracle.fill_ghosts(cfg, qj)
+    s = Solver(cfg)
+    s.set_state(qj)
+    a, b = s.rhs(), oracle.rhs(cfg, qj)
+    if visc == "LES":
+        assert np.abs(a - b).max() <= 1e-11 * np.abs(b).max()
+    else:
+        assert np.array_equal(a, b)
