@@ -46,17 +46,18 @@ int launch_one(const StepArgs<T>& A, int last, cudaStream_t s) {
   if (DIR == 0) grid = dim3((Nx + 31) / 32, (Ny + SWEEP_BR - 1) / SWEEP_BR, Nz);
   else if (DIR == 1) grid = dim3((Nx + 31) / 32, (Ny + SWEEP_BF - 1) / SWEEP_BF, Nz);
   else grid = dim3((Nx + 31) / 32, (Nz + SWEEP_BZ - 1) / SWEEP_BZ, Ny);
+  cudaError_t rc;
   if constexpr (TM) {
     // this direction's tile tensor maps from the handle (A.tmaps, a host address)
     SweepMaps maps;
     if (A.tmaps) std::memcpy(&maps, static_cast<const unsigned char*>(A.tmaps) + DIR * sizeof(SweepMaps),
                              sizeof(SweepMaps));
     else std::memset(&maps, 0, sizeof(SweepMaps));
-    k_sweep_tm<DIM, DIR, ORDER, VK, LES, T, SHARE><<<grid, block, smem, s>>>(A, last, maps, A.tmaps ? 1 : 0);
+    rc = launch_step(k_sweep_tm<DIM, DIR, ORDER, VK, LES, T, SHARE>, grid, block, smem, s, A, last, maps, A.tmaps ? 1 : 0);
   } else {
-    k_sweep<DIM, DIR, ORDER, VK, LES, T, SHARE><<<grid, block, smem, s>>>(A, last);
+    rc = launch_step(k_sweep<DIM, DIR, ORDER, VK, LES, T, SHARE>, grid, block, smem, s, A, last);
   }
-  return cudaPeekAtLastError() == cudaSuccess ? 0 : 1;
+  return rc == cudaSuccess ? 0 : 1;
 }
 
 template <int DIM, int ORDER, int VK, bool LES, class T>

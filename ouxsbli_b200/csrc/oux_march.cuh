@@ -72,6 +72,7 @@ __device__ __forceinline__ double load_early(const double* p) {
 
 template <int ORDER, int VK, bool LES, class T, bool SHARE>
 __global__ void __launch_bounds__(32 * MARCH_WARPS, ym_minb<T>()) k_march_y(StepArgs<T> A, int seg) {
+  step_begin();
   constexpr int DIR = 1, R = YM_R, MC = YM_C, NR = YM_RING, FS = NR * MC, NP = (R + 2) * MC;
   extern __shared__ __align__(16) unsigned char smraw[];
   const Geo& G = A.G;
@@ -202,8 +203,7 @@ int launch_march_y(const StepArgs<T>& A, cudaStream_t s) {
   const int seg = march_split(Ny, 148 * ym_minb<T>() * MARCH_WARPS, (int64_t)groups * Nz, 2.0,
                               [](int c) { return (c + YM_R) / YM_R; });
   const dim3 grid((unsigned)((groups + MARCH_WARPS - 1) / MARCH_WARPS), (unsigned)((Ny + seg - 1) / seg), (unsigned)Nz);
-  kern<<<grid, 32 * MARCH_WARPS, smem, s>>>(A, seg);
-  return cudaPeekAtLastError() == cudaSuccess ? 0 : 1;
+  return launch_step(kern, grid, dim3(32 * MARCH_WARPS), smem, s, A, seg) == cudaSuccess ? 0 : 1;
 }
 
 // ---- z sweep -----------------------------------------------------------------------
@@ -230,6 +230,7 @@ template <class T> __host__ __device__ constexpr int zm_minb() { return 4; }
 
 template <int ORDER, int VK, bool LES, class T, bool SHARE>
 __global__ void __launch_bounds__(32 * zm_warps<T>(), zm_minb<T>()) k_march_z(StepArgs<T> A, int seg) {
+  step_begin();
   constexpr int DIR = 2, NC = ZM_ROWS, NA = zm_aux_rows<SHARE>();
   constexpr bool MXC = sizeof(T) < sizeof(double);
   extern __shared__ __align__(16) unsigned char smraw[];
@@ -356,8 +357,7 @@ int launch_march_z(const StepArgs<T>& A, cudaStream_t s) {
   if (Nz <= 0) return 0;  // an empty part of a split stage
   const int groups = (Nx + 31) / 32, seg = march_split(Nz, 148 * zm_minb<T>() * zm_warps<T>(), (int64_t)groups * Ny, 4.0, [](int c) { return c; });
   const dim3 grid((unsigned)((groups + zm_warps<T>() - 1) / zm_warps<T>()), (unsigned)Ny, (unsigned)((Nz + seg - 1) / seg));
-  kern<<<grid, 32 * zm_warps<T>(), smem, s>>>(A, seg);
-  return cudaPeekAtLastError() == cudaSuccess ? 0 : 1;
+  return launch_step(kern, grid, dim3(32 * zm_warps<T>()), smem, s, A, seg) == cudaSuccess ? 0 : 1;
 }
 
 // ---- x sweep ---------------------------------------------------------------------
@@ -380,6 +380,7 @@ template <class T> __host__ __device__ constexpr int march_x_minb() { return 8; 
 
 template <int ORDER, int VK, bool LES, class T, bool SHARE>
 __global__ void __launch_bounds__(32 * MARCH_WARPS, march_x_minb<T>()) k_march_x(StepArgs<T> A, int nrow, int E) {
+  step_begin();
   constexpr int FS = XM_RING + 5, E0 = SHARE ? 2 : 0, CX = SHARE ? 3 : 5;
   extern __shared__ __align__(16) unsigned char smraw[];
   const Geo& G = A.G;
@@ -491,8 +492,7 @@ int launch_march_x(const StepArgs<T>& A, cudaStream_t s) {
                                            [&](int r) { return ((int64_t)r * E + 31) / 32; }));
   const int warps = (Ny + nrow - 1) / nrow;
   const dim3 grid((unsigned)((warps + MARCH_WARPS - 1) / MARCH_WARPS), (unsigned)Nz, 1);
-  kern<<<grid, 32 * MARCH_WARPS, smem, s>>>(A, nrow, E);
-  return cudaPeekAtLastError() == cudaSuccess ? 0 : 1;
+  return launch_step(kern, grid, dim3(32 * MARCH_WARPS), smem, s, A, nrow, E) == cudaSuccess ? 0 : 1;
 }
 
 template <int DIR, int ORDER, int VK, bool LES, class T, bool SHARE>

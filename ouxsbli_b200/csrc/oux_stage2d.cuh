@@ -49,6 +49,7 @@ template <int ORDER, bool KONLY, class T> __host__ __device__ constexpr size_t s
 template <int ORDER, bool KONLY, class T>
 __global__ void __launch_bounds__(S2_THREADS, KONLY ? 3 : 2)
 k_stage2d(StepArgs<T> A, const void* __restrict__ src, void* dst, double* keep) {
+  step_begin();
   constexpr bool MX = sizeof(T) < sizeof(double);
   constexpr int H = s2_halo<ORDER, KONLY>(), LX = S2_TX + 2 * H, LY = S2_TY + 2 * H, NC = LX * LY;
   constexpr int NFX = (S2_TX + 1) * S2_TY, NFY = S2_TX * (S2_TY + 1);
@@ -243,8 +244,7 @@ int launch_stage2d(const StepArgs<T>& A, const void* src, void* dst, double* kee
   if (attr != cudaSuccess) return 1;
   const Geo& G = A.G;
   const dim3 grid((unsigned)((G.nx - 2 * G.gx + S2_TX - 1) / S2_TX), (unsigned)((G.ny - 2 * G.gy + S2_TY - 1) / S2_TY));
-  kern<<<grid, S2_THREADS, smem, s>>>(A, src, dst, keep);
-  return cudaPeekAtLastError() == cudaSuccess ? 0 : 1;
+  return launch_step(kern, grid, dim3(S2_THREADS), smem, s, A, src, dst, keep) == cudaSuccess ? 0 : 1;
 }
 
 template <class T>

@@ -1351,6 +1351,7 @@ template <int DIM, int DIR, int VK> __host__ __device__ constexpr bool sweep_tma
 template <int DIM, int DIR, int ORDER, int VK, bool LES, class T, bool SHARE = false>
 __global__ void __launch_bounds__(sweep_threads<DIR>(), DIR == 0 ? OUX_SWEEP_MINB_X : OUX_SWEEP_MINB_YZ)
 k_sweep(StepArgs<T> A, int last) {
+  step_begin();
   extern __shared__ __align__(16) unsigned char smraw[];
   // coherent loads: measured as fast as the read-only path for y/z and faster for x
   constexpr int VB = vk_base(VK);
@@ -1366,6 +1367,7 @@ k_sweep(StepArgs<T> A, int last) {
 template <int DIM, int DIR, int ORDER, int VK, bool LES, class T, bool SHARE = false>
 __global__ void __launch_bounds__(sweep_threads<DIR>(), DIR == 0 ? OUX_SWEEP_MINB_X : OUX_SWEEP_MINB_YZ)
 k_sweep_tm(StepArgs<T> A, int last, const __grid_constant__ SweepMaps maps, int use) {
+  step_begin();
   extern __shared__ __align__(128) unsigned char smtile[];  // tensor copies land 128-byte aligned
   unsigned char* smraw = smtile;
   static_assert(sweep_tma<DIM, DIR, VK>(), "k_sweep_tm serves the TMA-staged sweeps");
