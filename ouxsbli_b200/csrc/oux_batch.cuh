@@ -122,7 +122,7 @@ __device__ __forceinline__ void batch_sweep(const StepArgs<T>& A, int last, int 
     int b0, b1, b2;
     if (DIR == 0) { b0 = t % n[0]; b1 = (t / n[0]) % n[1]; b2 = t / (n[0] * n[1]); }
     else { b1 = t % n[1]; b0 = (t / n[1]) % n[0]; b2 = t / (n[0] * n[1]); }  // pencil along the sweep
-    sweep_tile<DIM, DIR, ORDER, VK, LES, T, ROWS, false, KONLY>(A, last, b0, b1, b2, smraw, threadIdx.x,
+    sweep_tile<DIM, DIR, ORDER, VK, LES, T, ROWS, KONLY>(A, last, b0, b1, b2, smraw, threadIdx.x,
                                                               BATCH_THREADS);
     __syncthreads();
   }

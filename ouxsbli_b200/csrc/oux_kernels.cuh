@@ -107,9 +107,13 @@ template <class T> struct StepArgs {
 // kernel's blocks may be set up while the one before it drains.  step_begin, the first
 // thing each of them does, lets the next kernel's blocks be set up in turn and then
 // waits until every kernel before this one has finished and its writes are visible (each
-// of them having waited likewise).  It hides a launch's latency, 1 to 3 us, which counts on
-// small grids: measured on B200 (us per pass) 60^3 inviscid RK4 step 221 -> 184, four 64^3
-// SLAU-6 steps 1489 -> 1339, 81^3 LES step 541 -> 504, ten 513 x 7 steps 430 -> 382.
+// of them having waited likewise).  A kernel's lifetime so overlaps that of the kernel
+// that writes its inputs, so these kernels read with plain loads only: the read-only path
+// (ld.global.nc, from __ldg or const __restrict__ kernel parameters) wants data that nobody
+// writes while the kernel lives, and its loads may be moved above the wait.  The early
+// set-up hides a launch's latency, 1 to 3 us, which counts on small grids: measured on B200
+// (us per pass) 60^3 inviscid RK4 step 221 -> 184, four 64^3 SLAU-6 steps 1489 -> 1339, 81^3
+// LES step 541 -> 504, ten 513 x 7 steps 430 -> 382.
 __device__ __forceinline__ void step_begin() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -127,16 +131,6 @@ inline cudaError_t launch_step(void (*kernel)(P...), dim3 grid, dim3 block, size
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
-}
-
-// Load through the read-only data path when the caller guarantees the array is
-// not written during the kernel (RO = true: the single-solve kernels); plain
-// coherent load otherwise (the batched kernel, where other blocks of the same
-// launch produce the fields).
-template <bool RO, class T>
-__device__ __forceinline__ T ldro(const T* p) {
-  if constexpr (RO) return __ldg(p);
-  else return *p;
 }
 
 // Padded cell (i, j, k) of a flat index t (x fastest over nx, then ny, then nz).
@@ -195,37 +189,37 @@ __device__ __forceinline__ void prim_store(const double* q, double Jv, const Fie
   if constexpr (VISC) W.mu[o] = (T)(K.sutherland / (temp + 111.0) * (temp * sqrt(temp)));
 }
 
-template <int DIM, bool VISC, class TS, class T, bool RO = false>
+template <int DIM, bool VISC, class TS, class T>
 __device__ __forceinline__ void prim_cell(const TS* Q, const Geo& G, const Fields<T>& W, const double* jac,
                                           const PhysConst& K, int i, int j, int k) {
   static_assert(sizeof(T) == sizeof(double), "the mixed form decodes through prim_mx_cell");
   const int64_t o = G.at(i, j, k);
   double q[DIM + 2], v[3];
 #pragma unroll
-  for (int l = 0; l < DIM + 2; ++l) q[l] = (double)ldro<RO>(Q + o + l * G.vs);
-  prim_store<DIM, VISC, false>(q, ldro<RO>(jac + (int64_t)j * G.nx + i), W, o, K, v);
+  for (int l = 0; l < DIM + 2; ++l) q[l] = (double)Q[o + l * G.vs];
+  prim_store<DIM, VISC, false>(q, jac[(int64_t)j * G.nx + i], W, o, K, v);
 }
 
-template <int DIM, bool VISC, class TS, class T, bool RO = false>
+template <int DIM, bool VISC, class TS, class T>
 __device__ __forceinline__ void prim_cell(const TS* Q, const Geo& G, const Fields<T>& W, const double* jac,
                                           const PhysConst& K, int64_t t) {
   int i, j, k;
   cell_of(G, t, i, j, k);
-  prim_cell<DIM, VISC, TS, T, RO>(Q, G, W, jac, K, i, j, k);
+  prim_cell<DIM, VISC, TS, T>(Q, G, W, jac, K, i, j, k);
 }
 
 template <int DIM, bool VISC, class TS, class T>
-__global__ void __launch_bounds__(PLANE_THREADS) k_prim(const TS* __restrict__ Q, Geo G, Fields<T> W,
-                                                        const double* __restrict__ jac, PhysConst K) {
+__global__ void __launch_bounds__(PLANE_THREADS) k_prim(const TS* Q, Geo G, Fields<T> W,
+                                                        const double* jac, PhysConst K) {
   step_begin();
   int i, j, k;
-  if (plane_cell(G, i, j, k)) prim_cell<DIM, VISC, TS, T, true>(Q, G, W, jac, K, i, j, k);
+  if (plane_cell(G, i, j, k)) prim_cell<DIM, VISC, TS, T>(Q, G, W, jac, K, i, j, k);
 }
 
 // ---- mixed-form primitives: Q = Q^n (FP64) + dQ (FP32 stage increment, may be
 // null), evaluated in FP64 like k_prim, stored in FP32 with p and T as deviations
 // from the per-solve references K.p_ref, K.T_ref.
-template <int DIM, bool VISC, bool RO = false>
+template <int DIM, bool VISC>
 __device__ __forceinline__ void prim_mx_cell(const double* Qn, const float* dQ, const Geo& G,
                                              const Fields<float>& W, const double* jac, const PhysConst& K,
                                              int i, int j, int k) {
@@ -233,27 +227,27 @@ __device__ __forceinline__ void prim_mx_cell(const double* Qn, const float* dQ, 
   double q[5];
 #pragma unroll
   for (int l = 0; l < DIM + 2; ++l)
-    q[l] = ldro<RO>(Qn + o + l * G.vs) + (dQ ? (double)ldro<RO>(dQ + o + l * G.vs) : 0.0);
+    q[l] = Qn[o + l * G.vs] + (dQ ? (double)dQ[o + l * G.vs] : 0.0);
   double v[3];
-  prim_store<DIM, VISC, true>(q, ldro<RO>(jac + (int64_t)j * G.nx + i), W, o, K, v);
+  prim_store<DIM, VISC, true>(q, jac[(int64_t)j * G.nx + i], W, o, K, v);
 }
 
-template <int DIM, bool VISC, bool RO = false>
+template <int DIM, bool VISC>
 __device__ __forceinline__ void prim_mx_cell(const double* Qn, const float* dQ, const Geo& G,
                                              const Fields<float>& W, const double* jac, const PhysConst& K,
                                              int64_t t) {
   int i, j, k;
   cell_of(G, t, i, j, k);
-  prim_mx_cell<DIM, VISC, RO>(Qn, dQ, G, W, jac, K, i, j, k);
+  prim_mx_cell<DIM, VISC>(Qn, dQ, G, W, jac, K, i, j, k);
 }
 
 template <int DIM, bool VISC>
-__global__ void __launch_bounds__(PLANE_THREADS) k_prim_mx(const double* __restrict__ Qn,
-                                                           const float* __restrict__ dQ, Geo G, Fields<float> W,
-                                                           const double* __restrict__ jac, PhysConst K) {
+__global__ void __launch_bounds__(PLANE_THREADS) k_prim_mx(const double* Qn, const float* dQ, Geo G,
+                                                           Fields<float> W,
+                                                           const double* jac, PhysConst K) {
   step_begin();
   int i, j, k;
-  if (plane_cell(G, i, j, k)) prim_mx_cell<DIM, VISC, true>(Qn, dQ, G, W, jac, K, i, j, k);
+  if (plane_cell(G, i, j, k)) prim_mx_cell<DIM, VISC>(Qn, dQ, G, W, jac, K, i, j, k);
 }
 
 // ---- Ducros sensor: calc_Ducros (3D_solver/src/calc_hybrid.f90:11-72; 2D twin
@@ -319,7 +313,7 @@ __device__ __forceinline__ void sensor_of_diffs(const Geo& G, const Fields<T>& W
   }
 }
 
-template <int DIM, class T, bool RO = false>
+template <int DIM, class T>
 __device__ __forceinline__ void sensor_cell(const Geo& G, const Fields<T>& W, const Metrics& M, int i, int j,
                                             int k) {
   if (i < 1 || i > G.nx - 2 || j < 1 || j > G.ny - 2) return;
@@ -328,22 +322,22 @@ __device__ __forceinline__ void sensor_cell(const Geo& G, const Fields<T>& W, co
   const T* vel[3] = {W.u, W.v, W.w};
   const int64_t st[3] = {1, G.sx, G.plane};
   sensor_of_diffs<DIM, T>(G, W, M, i, j, k, [&](int c, int a) -> T {
-    return -ldro<RO>(vel[c] + o - st[a]) + ldro<RO>(vel[c] + o + st[a]);
+    return -vel[c][o - st[a]] + vel[c][o + st[a]];
   });
 }
 
-template <int DIM, class T, bool RO = false>
+template <int DIM, class T>
 __device__ __forceinline__ void sensor_cell(const Geo& G, const Fields<T>& W, const Metrics& M, int64_t t) {
   int i, j, k;
   cell_of(G, t, i, j, k);
-  sensor_cell<DIM, T, RO>(G, W, M, i, j, k);
+  sensor_cell<DIM, T>(G, W, M, i, j, k);
 }
 
 template <int DIM, class T>
 __global__ void __launch_bounds__(PLANE_THREADS) k_sensor(Geo G, Fields<T> W, Metrics M) {
   step_begin();
   int i, j, k;
-  if (plane_cell(G, i, j, k)) sensor_cell<DIM, T, false>(G, W, M, i, j, k);
+  if (plane_cell(G, i, j, k)) sensor_cell<DIM, T>(G, W, M, i, j, k);
 }
 
 // Mixed form: the sensor from FP64 velocities decoded from Q^n + the FP32 stage
@@ -353,7 +347,7 @@ __global__ void __launch_bounds__(PLANE_THREADS) k_sensor(Geo G, Fields<T> W, Me
 // them into much larger relative errors of the divergence; this way the sensor is the
 // FP64 solve's value for the same state to within one FP32 rounding, so the hybrid
 // threshold and the TVD switch flip only where a face value lies that close to 0.4.
-template <int DIM, bool RO = false>
+template <int DIM>
 __device__ __forceinline__ void sensor_mx_cell(const Geo& G, const double* Qn, const float* dQ,
                                                const Fields<float>& W, const Metrics& M, int i, int j, int k) {
   if (i < 1 || i > G.nx - 2 || j < 1 || j > G.ny - 2) return;
@@ -361,7 +355,7 @@ __device__ __forceinline__ void sensor_mx_cell(const Geo& G, const double* Qn, c
   const int64_t o = G.at(i, j, k);
   auto q = [&](int64_t c, int l) -> double {
     const int64_t a = c + l * G.vs;
-    return ldro<RO>(Qn + a) + (dQ ? (double)ldro<RO>(dQ + a) : 0.0);
+    return Qn[a] + (dQ ? (double)dQ[a] : 0.0);
   };
   // velocities of cell c (prim_mx_cell: over = 1 / q0, u = q1 * over)
   auto vel = [&](int64_t c, double (&v)[3]) {
@@ -406,21 +400,20 @@ __device__ __forceinline__ void sensor_mx_cell(const Geo& G, const double* Qn, c
   }
 }
 
-template <int DIM, bool RO = false>
+template <int DIM>
 __device__ __forceinline__ void sensor_mx_cell(const Geo& G, const double* Qn, const float* dQ,
                                                const Fields<float>& W, const Metrics& M, int64_t t) {
   int i, j, k;
   cell_of(G, t, i, j, k);
-  sensor_mx_cell<DIM, RO>(G, Qn, dQ, W, M, i, j, k);
+  sensor_mx_cell<DIM>(G, Qn, dQ, W, M, i, j, k);
 }
 
 template <int DIM>
-__global__ void __launch_bounds__(PLANE_THREADS) k_sensor_mx(Geo G, const double* __restrict__ Qn,
-                                                             const float* __restrict__ dQ, Fields<float> W,
-                                                             Metrics M) {
+__global__ void __launch_bounds__(PLANE_THREADS) k_sensor_mx(Geo G, const double* Qn, const float* dQ,
+                                                             Fields<float> W, Metrics M) {
   step_begin();
   int i, j, k;
-  if (plane_cell(G, i, j, k)) sensor_mx_cell<DIM, true>(G, Qn, dQ, W, M, i, j, k);
+  if (plane_cell(G, i, j, k)) sensor_mx_cell<DIM>(G, Qn, dQ, W, M, i, j, k);
 }
 
 // ---- primitives and Ducros sensor in one pass (3D) --------------------------------
@@ -452,8 +445,8 @@ inline dim3 prim_fused_grid(const Geo& G) {
 }
 
 template <bool VISC, bool MX, class TS, class T>
-__global__ void __launch_bounds__(PS_TX * PS_TY, 4) k_prim_fused(const TS* __restrict__ Q, const float* __restrict__ dQ,
-                                                              Geo G, Fields<T> W, Metrics M, PhysConst K) {
+__global__ void __launch_bounds__(PS_TX * PS_TY, 4) k_prim_fused(const TS* Q, const float* dQ, Geo G,
+                                                              Fields<T> W, Metrics M, PhysConst K) {
   step_begin();
   constexpr int RX = PS_TX + 2, RY = PS_TY + 2, RZ = PS_TZ + 2, RN = RX * RY * RZ;
   extern __shared__ __align__(16) unsigned char smraw[];
@@ -472,12 +465,12 @@ __global__ void __launch_bounds__(PS_TX * PS_TY, 4) k_prim_fused(const TS* __res
 #pragma unroll
     for (int l = 0; l < 5; ++l) {
       if (l == 4 && !own) break;
-      q[l] = (double)__ldg(Q + o + l * G.vs);
-      if constexpr (MX) q[l] = q[l] + (dQ ? (double)__ldg(dQ + o + l * G.vs) : 0.0);
+      q[l] = (double)Q[o + l * G.vs];
+      if constexpr (MX) q[l] = q[l] + (dQ ? (double)dQ[o + l * G.vs] : 0.0);
     }
     double v[3];
     if (own) {
-      prim_store<3, VISC, MX>(q, __ldg(M.jac + (int64_t)j * G.nx + i), W, o, K, v);
+      prim_store<3, VISC, MX>(q, M.jac[(int64_t)j * G.nx + i], W, o, K, v);
     } else {
       const double over = 1.0 / q[0];
       v[0] = q[1] * over;
@@ -568,23 +561,24 @@ __global__ void __launch_bounds__(PLANE_THREADS, 8) k_grad(Geo G, Fields<T> W, M
     const T inv = fits ? (T)invd[a][c[a]] : T(0);
     const T sc = sens ? ducros_scale<T>(invd[a], c[a]) : T(0);
     T d[3];  // (-vel_q(o - st_a) + vel_q(o + st_a)) times the sensor's scale
+    T gq[3] = {};  // stored after the three components' loads: a load may not pass a store
 #pragma unroll
     for (int q = 0; q < 3; ++q) {
       const T* f = vel[q] + o;
-      T gq = T(0);
       d[q] = T(0);
       if (fits) {
-        const T m1 = __ldg(f - st[a]), p1 = __ldg(f + st[a]);
-        const T m2 = __ldg(f - 2 * st[a]), p2 = __ldg(f + 2 * st[a]);
+        const T m1 = f[-st[a]], p1 = f[st[a]];
+        const T m2 = f[-2 * st[a]], p2 = f[2 * st[a]];
         T m3 = T(0), p3 = T(0);
-        if constexpr (SIXTH) { m3 = __ldg(f - 3 * st[a]); p3 = __ldg(f + 3 * st[a]); }
-        gq = node_deriv_of<SIXTH, T>(m3, m2, m1, p1, p2, p3, inv);
+        if constexpr (SIXTH) { m3 = f[-3 * st[a]]; p3 = f[3 * st[a]]; }
+        gq[q] = node_deriv_of<SIXTH, T>(m3, m2, m1, p1, p2, p3, inv);
         if (sens) d[q] = (-m1 + p1) * sc;
       } else if (sens) {
-        d[q] = (-__ldg(f - st[a]) + __ldg(f + st[a])) * sc;
+        d[q] = (-f[-st[a]] + f[st[a]]) * sc;
       }
-      W.grad[3 * q + a][o] = gq;
     }
+#pragma unroll
+    for (int q = 0; q < 3; ++q) W.grad[3 * q + a][o] = gq[q];
     if constexpr (SENSOR) {
       if (a == 0) { div = d[0]; r3 = d[1]; dwdx = d[2]; }                  // dudx, dvdx, dwdx
       else if (a == 1) { div = div + d[1]; r3 = r3 - d[0]; dwdy = d[2]; }  // + dvdy; dvdx - dudy

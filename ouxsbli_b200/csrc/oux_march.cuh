@@ -141,7 +141,7 @@ __global__ void __launch_bounds__(32 * MARCH_WARPS, ym_minb<T>()) k_march_y(Step
     T F[5] = {};
     if (valid) {
       const int fc[3] = {i, f, k};
-      face_flux<3, DIR, ORDER, VK, LES, T, false, false, SHARE>(A, st0, fc, F);
+      face_flux<3, DIR, ORDER, VK, LES, T, false, SHARE>(A, st0, fc, F);
     }
     if constexpr (SHARE) {
       __syncwarp();  // the chunk's positions are written
@@ -317,7 +317,7 @@ __global__ void __launch_bounds__(32 * zm_warps<T>(), zm_minb<T>()) k_march_z(St
     if (xok && f >= f0) {
       T F[5];
       const int fc[3] = {i, t, f};
-      face_flux<3, DIR, ORDER, VK, LES, T, false, false, SHARE>(A, st0, fc, F);
+      face_flux<3, DIR, ORDER, VK, LES, T, false, SHARE>(A, st0, fc, F);
       if constexpr (SHARE) {
         auto P = [&](int k, int m) -> T { return m == 0 ? P0[k] : m == 1 ? P1[k] : v[k]; };
         T vo[4];
@@ -444,7 +444,7 @@ __global__ void __launch_bounds__(32 * MARCH_WARPS, march_x_minb<T>()) k_march_x
     T F[5] = {};
     if (valid) {
       const int fc[3] = {f, j, k};
-      face_flux<3, 0, ORDER, VK, LES, T, false, false, SHARE>(A, st0, fc, F);
+      face_flux<3, 0, ORDER, VK, LES, T, false, SHARE>(A, st0, fc, F);
     }
     if constexpr (SHARE) {
       __syncwarp();

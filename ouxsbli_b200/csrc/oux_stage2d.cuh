@@ -48,7 +48,7 @@ template <int ORDER, bool KONLY, class T> __host__ __device__ constexpr size_t s
 // a copy of Q^n the later stages read, so that the last one can write the state in place.
 template <int ORDER, bool KONLY, class T>
 __global__ void __launch_bounds__(S2_THREADS, KONLY ? 3 : 2)
-k_stage2d(StepArgs<T> A, const void* __restrict__ src, void* dst, double* keep) {
+k_stage2d(StepArgs<T> A, const void* src, void* dst, double* keep) {
   step_begin();
   constexpr bool MX = sizeof(T) < sizeof(double);
   constexpr int H = s2_halo<ORDER, KONLY>(), LX = S2_TX + 2 * H, LY = S2_TY + 2 * H, NC = LX * LY;
@@ -84,19 +84,31 @@ k_stage2d(StepArgs<T> A, const void* __restrict__ src, void* dst, double* keep) 
   }
   cp_async_commit();
 
-  // ---- primitives of the tile and its halo (prim_cell / prim_mx_cell) ----
-  for (int c = tid; c < NC; c += S2_THREADS) {
+  // ---- primitives of the tile and its halo (prim_cell / prim_mx_cell); a thread's loads
+  // all go out before its first store ----
+  constexpr int ND = (NC + S2_THREADS - 1) / S2_THREADS;  // cells a thread decodes
+  double q[ND][4], Jv[ND];
+  bool in[ND];
+#pragma unroll
+  for (int n = 0; n < ND; ++n) {
+    const int c = tid + n * S2_THREADS;
     const int i = bx - H + c % LX, j = by - H + c / LX;
-    if (i < 0 || i >= G.nx || j < 0 || j >= G.ny || i >= ex + H || j >= ey + H) continue;
+    in[n] = c < NC && i >= 0 && i < min(G.nx, ex + H) && j >= 0 && j < min(G.ny, ey + H);
+    if (!in[n]) continue;
     const int64_t o = G.at(i, j, 0);
-    double q[4];
+    Jv[n] = A.M.jac[(int64_t)j * G.nx + i];
 #pragma unroll
     for (int l = 0; l < 4; ++l) {
-      if constexpr (MX) q[l] = A.Qn[o + l * G.vs] + (Sf ? (double)__ldg(Sf + o + l * G.vs) : 0.0);
-      else q[l] = __ldg(Sd + o + l * G.vs);
+      if constexpr (MX) q[n][l] = A.Qn[o + l * G.vs] + (Sf ? (double)Sf[o + l * G.vs] : 0.0);
+      else q[n][l] = Sd[o + l * G.vs];
     }
+  }
+#pragma unroll
+  for (int n = 0; n < ND; ++n) {
+    if (!in[n]) continue;
+    const int c = tid + n * S2_THREADS;
     double v[3], rho, p, temp;
-    prim_decode<2>(q, __ldg(A.M.jac + (int64_t)j * G.nx + i), A.K, rho, v, p, temp);
+    prim_decode<2>(q[n], Jv[n], A.K, rho, v, p, temp);
     tile[c] = (T)rho;
     tile[NC + c] = (T)v[0];
     tile[2 * NC + c] = (T)v[1];
@@ -138,7 +150,7 @@ k_stage2d(StepArgs<T> A, const void* __restrict__ src, void* dst, double* keep) 
     };
     const int fc[3] = {fi, fj, 0};
     T F[5];
-    face_flux<2, D, ORDER, VK_EULER, false, T, false, KONLY, false>(A, st0, fc, F);
+    face_flux<2, D, ORDER, VK_EULER, false, T, KONLY, false>(A, st0, fc, F);
     out[0] = (double)F[0];
     out[stride] = (double)F[1];
     out[2 * stride] = (double)F[2];

@@ -170,9 +170,9 @@ struct SweepMaps {
 constexpr int TMA_WAIT_LIMIT = 1 << 20;
 
 // transverse node derivative of `a` along axis `ax` at offset o (4th/6th order)
-template <bool SIXTH, bool RO, class T>
+template <bool SIXTH, class T>
 __device__ __forceinline__ T node_d(const T* a, int64_t o, int64_t st, T inv) {
-  auto A = [&](int64_t q) { return ldro<RO>(a + q); };
+  auto A = [&](int64_t q) { return a[q]; };
   if constexpr (SIXTH)
     return (T(1.0 / 60.0) * (-A(o - 3 * st) + A(o + 3 * st)) + T(0.15) * (A(o - 2 * st) - A(o + 2 * st)) +
             T(0.75) * (-A(o - st) + A(o + st))) * inv;
@@ -498,17 +498,10 @@ __device__ __forceinline__ void me4_face(const StepArgs<T>& A, const PosAcc& P, 
 
 // ---- Gaitonde-Visbal 2nd order: 3D_solver/src/calc_visc2.f90.fypp (2D :10-103) ----
 // Reads global arrays directly: face between o and o + st[nd].
-template <int DIM, bool LES, bool RO, class T>
+template <int DIM, bool LES, class T>
 __device__ __forceinline__ void visc_gv2(const StepArgs<T>& A, int nd, int64_t o, const int64_t st[3],
                                          const T invs[3], T out[4]) {
-  // read-only view of the fields: W.f[q] loads through ldro<RO>
-  struct RoField {
-    const T* p;
-    __device__ T operator[](int64_t q) const { return ldro<RO>(p + q); }
-  };
-  struct {
-    RoField u, v, w, mu, T_, mut, qc2;
-  } W{{A.W.u}, {A.W.v}, {A.W.w}, {A.W.mu}, {A.W.T_}, {A.W.mut}, {A.W.qc2}};
+  const Fields<T>& W = A.W;
   const int64_t o2 = o + st[nd];
   const T inv = invs[nd];
   auto vel = [&](int c, int64_t q) -> T { return c == 0 ? W.u[q] : (c == 1 ? W.v[q] : (DIM == 3 ? W.w[q] : T(0))); };
@@ -529,7 +522,7 @@ __device__ __forceinline__ void visc_gv2(const StepArgs<T>& A, int nd, int64_t o
     for (int c = 0; c < 3; ++c) sg[c] = msd * (-vel(c, o) + vel(c, o2));
   }
   auto cross = [&](bool sgs, int c, int t) -> T {
-    const RoField m = sgs ? W.mut : W.mu;
+    const T* m = sgs ? W.mut : W.mu;
     const int64_t s = st[t];
     T m1 = T(0.0625) * (m[o - s] + m[o] + m[o2 - s] + m[o2]);
     T m2 = T(0.0625) * (m[o] + m[o + s] + m[o2] + m[o2 + s]);
@@ -767,7 +760,7 @@ namespace oux {
 // Flux of the face whose left cell is fc (padded indices): the convective flux and,
 // unless the caller combines shared ME4 positions itself (SHARE), minus the viscous one.
 // st0(field, m) reads the tile field of cell f - 2 + m along DIR, m = 0 .. 5.
-template <int DIM, int DIR, int ORDER, int VK, bool LES, class T, bool RO, bool KONLY, bool SHARE, class Acc>
+template <int DIM, int DIR, int ORDER, int VK, bool LES, class T, bool KONLY, bool SHARE, class Acc>
 __device__ __forceinline__ void face_flux(const StepArgs<T>& A, const Acc& st0, const int fc[3], T F[5]) {
   constexpr int H = ORDER / 2;
   constexpr int VB = vk_base(VK);
@@ -809,7 +802,7 @@ __device__ __forceinline__ void face_flux(const StepArgs<T>& A, const Acc& st0, 
     if constexpr (VB == VK_GV2) {
       const int64_t o = G.at(fc[0], fc[1], DIM == 3 ? fc[2] : 0);
       T invs[3] = {(T)A.M.inv_dx[fc[0]], (T)A.M.inv_dy[fc[1]], DIM == 3 ? (T)A.M.inv_dz[fc[2]] : T(0)};
-      visc_gv2<DIM, LES, RO>(A, DIR, o, stv, invs, vo);
+      visc_gv2<DIM, LES>(A, DIR, o, stv, invs, vo);
     } else if constexpr (VK == VK_2D4) {
       // inner guard of calc_Ev4 / calc_Fv4 (2D): face 2..n-4, transverse 2..n-3
       const int nt = DIR == 0 ? G.ny : G.nx;
@@ -955,7 +948,7 @@ __device__ __forceinline__ void combine_cell(const StepArgs<T>& A, int i, int j,
 // one thread stages every field by a tensor copy completing one mbarrier, else the
 // threads fill the same layout with cp.async.
 template <int DIM, int DIR, int ORDER, int VK, bool LES, class T, int ROWS = default_rows<DIR>(),
-          bool RO = false, bool KONLY = false, int PF = 0, bool SHARE = false, bool GR = false, bool AT = false,
+          bool KONLY = false, int PF = 0, bool SHARE = false, bool GR = false, bool AT = false,
           bool TM = false>
 __device__ __forceinline__ void sweep_tile(const StepArgs<T>& A, int last, int b0, int b1, int b2,
                                            unsigned char* smraw, int tid, int nthr_all,
@@ -1123,27 +1116,27 @@ __device__ __forceinline__ void sweep_tile(const StepArgs<T>& A, int last, int b
       if constexpr (!HIGH || GR) continue;
     }
     if constexpr (!AT) {
-      tile[TF_RHO * FS + sl] = ldro<RO>(A.W.rho + o);
-      tile[TF_U * FS + sl] = ldro<RO>(A.W.u + o);
-      tile[TF_V * FS + sl] = ldro<RO>(A.W.v + o);
-      tile[TF_W * FS + sl] = (DIM == 3) ? ldro<RO>(A.W.w + o) : T(0);
-      tile[TF_P * FS + sl] = ldro<RO>(A.W.p + o);
-      tile[TF_T * FS + sl] = ldro<RO>(A.W.T_ + o);
-      if (!KONLY && A.scheme != 0) tile[TF_SEN * FS + sl] = ldro<RO>(A.W.sensor + o);
-      if constexpr (VK != VK_EULER) tile[TF_MU * FS + sl] = ldro<RO>(A.W.mu + o);
+      tile[TF_RHO * FS + sl] = A.W.rho[o];
+      tile[TF_U * FS + sl] = A.W.u[o];
+      tile[TF_V * FS + sl] = A.W.v[o];
+      tile[TF_W * FS + sl] = (DIM == 3) ? A.W.w[o] : T(0);
+      tile[TF_P * FS + sl] = A.W.p[o];
+      tile[TF_T * FS + sl] = A.W.T_[o];
+      if (!KONLY && A.scheme != 0) tile[TF_SEN * FS + sl] = A.W.sensor[o];
+      if constexpr (VK != VK_EULER) tile[TF_MU * FS + sl] = A.W.mu[o];
       if constexpr (LES) {
-        tile[TF_MUT * FS + sl] = ldro<RO>(A.W.mut + o);
-        tile[TF_QC2 * FS + sl] = ldro<RO>(A.W.qc2 + o);
+        tile[TF_MUT * FS + sl] = A.W.mut[o];
+        tile[TF_QC2 * FS + sl] = A.W.qc2[o];
       }
     }
     if constexpr (HIGH && GR) {  // transverse node derivatives from the gradient fields
       static_assert(DIM == 3, "gradient fields are built for 3D grids");
       constexpr int n = DIR, a1 = (n + 1) % 3, a2 = (n + 2) % 3;
       constexpr int ca = n == 0 ? 1 : 0, cb = n == 2 ? 1 : 2;
-      tile[TF_D0 * FS + sl] = ldro<RO>(A.W.grad[3 * a1 + a1] + o);
-      tile[TF_D1 * FS + sl] = ldro<RO>(A.W.grad[3 * a2 + a2] + o);
-      tile[TF_D2 * FS + sl] = ldro<RO>(A.W.grad[3 * n + ca] + o);
-      tile[TF_D3 * FS + sl] = ldro<RO>(A.W.grad[3 * n + cb] + o);
+      tile[TF_D0 * FS + sl] = A.W.grad[3 * a1 + a1][o];
+      tile[TF_D1 * FS + sl] = A.W.grad[3 * a2 + a2][o];
+      tile[TF_D2 * FS + sl] = A.W.grad[3 * n + ca][o];
+      tile[TF_D3 * FS + sl] = A.W.grad[3 * n + cb][o];
     } else if constexpr (HIGH) {  // transverse node derivatives (the viscous loaders' stencils)
       const T* vel[3] = {A.W.u, A.W.v, A.W.w};
       const double* invd[3] = {A.M.inv_dx, A.M.inv_dy, A.M.inv_dz};
@@ -1157,7 +1150,7 @@ __device__ __forceinline__ void sweep_tile(const StepArgs<T>& A, int last, int b
         const int na[3] = {G.nx, G.ny, G.nz};
         auto nd = [&](const T* f, int ax) -> T {
           if (WALL && !(ci[ax] >= HD && ci[ax] + HD < na[ax])) return T(0);
-          return node_d<SIXTH, RO>(f, o, stv[ax], (T)invd[ax][ci[ax]]);
+          return node_d<SIXTH>(f, o, stv[ax], (T)invd[ax][ci[ax]]);
         };
         tile[TF_D0 * FS + sl] = nd(vel[a1], a1);
         tile[TF_D1 * FS + sl] = nd(vel[a2], a2);
@@ -1170,8 +1163,8 @@ __device__ __forceinline__ void sweep_tile(const StepArgs<T>& A, int last, int b
         const int n = DIR, t = 1 - DIR;
         constexpr int HD = SIXTH ? 3 : 2;
         if (ci[t] >= HD && ci[t] + HD < (t == 0 ? G.nx : G.ny)) {
-          tile[TF_D0 * FS + sl] = node_d<SIXTH, RO>(vel[t], o, stv[t], (T)invd[t][ci[t]]);
-          tile[TF_D2 * FS + sl] = node_d<SIXTH, RO>(vel[n], o, stv[t], (T)invd[t][ci[t]]);
+          tile[TF_D0 * FS + sl] = node_d<SIXTH>(vel[t], o, stv[t], (T)invd[t][ci[t]]);
+          tile[TF_D2 * FS + sl] = node_d<SIXTH>(vel[n], o, stv[t], (T)invd[t][ci[t]]);
         } else {
           tile[TF_D0 * FS + sl] = T(0);
           tile[TF_D2 * FS + sl] = T(0);
@@ -1242,7 +1235,7 @@ __device__ __forceinline__ void sweep_tile(const StepArgs<T>& A, int last, int b
       T F[5];
       // tile position of cell f + off is base + (2 + off) * step
       auto st0 = [&](int field, int m) -> T { return tile[field * FS + base + m * step]; };
-      face_flux<DIM, DIR, ORDER, VK, LES, T, RO, KONLY, SHARE>(A, st0, fc, F);
+      face_flux<DIM, DIR, ORDER, VK, LES, T, KONLY, SHARE>(A, st0, fc, F);
 #pragma unroll
       for (int l = 0; l < 5; ++l) Fs[l * (TX * TY) + tid] = (double)F[l];
     }
@@ -1353,11 +1346,10 @@ __global__ void __launch_bounds__(sweep_threads<DIR>(), DIR == 0 ? OUX_SWEEP_MIN
 k_sweep(StepArgs<T> A, int last) {
   step_begin();
   extern __shared__ __align__(16) unsigned char smraw[];
-  // coherent loads: measured as fast as the read-only path for y/z and faster for x
   constexpr int VB = vk_base(VK);
   constexpr bool HIGH = (VB == VK_C6 || VB == VK_C4 || VB == VK_ME4 || VB == VK_2D4);
   constexpr bool GR = sweep_uses_grads<DIM, VK>();
-  sweep_tile<DIM, DIR, ORDER, VK, LES, T, default_rows<DIR>(), false, false, sweep_pf_mode<DIM, DIR, T>(), SHARE,
+  sweep_tile<DIM, DIR, ORDER, VK, LES, T, default_rows<DIR>(), false, sweep_pf_mode<DIM, DIR, T>(), SHARE,
              GR, !HIGH || GR, sweep_tma<DIM, DIR, VK>()>(A, last, blockIdx.x, blockIdx.y, blockIdx.z, smraw,
                                                         threadIdx.x, sweep_threads<DIR>());
 }
@@ -1371,7 +1363,7 @@ k_sweep_tm(StepArgs<T> A, int last, const __grid_constant__ SweepMaps maps, int 
   extern __shared__ __align__(128) unsigned char smtile[];  // tensor copies land 128-byte aligned
   unsigned char* smraw = smtile;
   static_assert(sweep_tma<DIM, DIR, VK>(), "k_sweep_tm serves the TMA-staged sweeps");
-  sweep_tile<DIM, DIR, ORDER, VK, LES, T, default_rows<DIR>(), false, false, sweep_pf_mode<DIM, DIR, T>(), SHARE,
+  sweep_tile<DIM, DIR, ORDER, VK, LES, T, default_rows<DIR>(), false, sweep_pf_mode<DIM, DIR, T>(), SHARE,
              true, true, true>(A, last, blockIdx.x, blockIdx.y, blockIdx.z, smraw, threadIdx.x, sweep_threads<DIR>(),
                                use ? &maps : nullptr);
 }

@@ -222,3 +222,26 @@ def test_tma_tile_geometry_meets_the_tensor_copy_rules():
                 y0 = bx0 - gx
                 assert y0 * elem % 16 == 0 and y0 >= 0
                 assert bx0 - y0 == gx and (bx0 + 31) - y0 < const["TMA_ROW"]
+
+
+def test_step_kernels_wait_first_and_load_plainly():
+    """Kernels launched with programmatic stream serialisation (launch_step) overlap the
+    kernel that writes their inputs: each calls step_begin before anything else, and none
+    reads through the read-only path (__ldg, ld.global.nc, const __restrict__ parameters),
+    which has no order with the wait.  Read from the sources."""
+    csrc = HEADER.parents[1] / "ouxsbli_b200" / "csrc"
+    text = {p.name: re.sub(r"//[^\n]*", "", p.read_text()) for p in csrc.glob("*.cu*")}
+    launched = {k for t in text.values() for k in re.findall(r"launch_step\(\s*(k_\w+)", t)}
+    launched |= {k for t in text.values() if "launch_step(kern" in t for k in re.findall(r"auto kern = (k_\w+)", t)}
+    assert {"k_prim", "k_prim_fused", "k_grad", "k_mut", "k_ghost", "k_sweep", "k_sweep_tm", "k_march_x", "k_march_y",
+            "k_march_z", "k_stage2d"} <= launched
+    found = set()
+    for name, t in text.items():
+        # the headers of these kernels hold nothing but their code and what they call
+        if any(re.search(rf"\b{k}\(", t) and "__global__" in t and name.endswith(".cuh") for k in launched):
+            assert not re.search(r"__ldg|ld\.global\.nc|__restrict__|__ldcs|__ldlu", t), name
+        for m in re.finditer(r"__global__[^{;]*?\b(k_\w+)\s*\([^{]*\)\s*\{\s*([^;]*;)", t):
+            if m.group(1) in launched:
+                found.add(m.group(1))
+                assert m.group(2) == "step_begin();", m.group(1)
+    assert found == launched

@@ -90,6 +90,24 @@ def test_sgs_viscosity_tiles(n, stretch):
     assert np.abs(a - b).max() <= 1e-11 * np.abs(b).max()
 
 
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("n", [(2, 1, 3), (3, 3, 1), (2, 1, 1), (33, 1, 5)])
+def test_sgs_edges_of_axes_of_one_cell(n, precision):
+    """Order 2: the only interior cell of a periodic axis of three is the source of both
+    its edges.  The fields hold NaN beforehand, so that a cell nobody writes shows."""
+    from ouxsbli_b200.solver import Solver
+    cfg, qj = box(n, order=2, scheme="SLAU", visc="LES", precision=precision)
+    s = Solver(cfg)
+    s.set_state(qj)
+    s.scratch[:10 * s.layout.var_stride // (1 if precision == "fp64" else 2)] = float("nan")
+    a, b = (rhs_interior(r, cfg.g, 3) for r in (s.rhs(), oracle.rhs(cfg, qj)))
+    if precision == "fp64":
+        assert np.abs(a - b).max() <= 1e-11 * np.abs(b).max()
+    else:
+        for l in range(5):
+            assert np.abs(a[:, l] - b[:, l]).max() <= 2e-6 * np.abs(qj[:, l]).max()
+
+
 def box2d(n, order, bc_x=0, bc_y=0, seed=0, boundary=None, **kw):
     """Smooth seeded 2D field on n = (x, y) interior cells."""
     rng = np.random.default_rng(seed)
