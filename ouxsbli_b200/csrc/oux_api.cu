@@ -613,13 +613,20 @@ int run_stage(oux_handle* h, const TS* src, StepArgs<T> A, cudaStream_t s) {
     }
   }
   if (h->les) {
-    Timed tm(h, KK_MUT, s);
-    constexpr size_t smem = mut_smem<T>();
-    static const cudaError_t attr =
-        cudaFuncSetAttribute(k_mut<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (attr != cudaSuccess) return fail(OUX_E_CUDA, "SGS viscosity pass: shared memory");
-    launch_step(k_mut<T>, mut_grid(G), dim3(MUT_TX * MUT_TY), smem, s, G, W, h->M, h->K);
-    h->launches++;
+    {
+      Timed tm(h, KK_MUT, s);
+      constexpr size_t smem = mut_smem<T>();
+      static const cudaError_t attr =
+          cudaFuncSetAttribute(k_mut<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      if (attr != cudaSuccess) return fail(OUX_E_CUDA, "SGS viscosity pass: shared memory");
+      launch_step(k_mut<T>, mut_grid(G), dim3(MUT_TX * MUT_TY), smem, s, G, W, h->M, h->K);
+      h->launches++;
+    }
+    if (mut_needs_edges(G)) {
+      Timed tm(h, KK_MUT_EDGES, s);
+      launch_step(k_mut_edges<T>, grid_for((int64_t)G.nx * G.ny * G.nz, 256), dim3(256), 0, s, G, W);
+      h->launches++;
+    }
   }
   int rc;
   if (h->profiling) {

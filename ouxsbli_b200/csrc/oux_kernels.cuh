@@ -740,7 +740,8 @@ __global__ void __launch_bounds__(MUT_TX * MUT_TY) k_mut(Geo G, Fields<T> W, Met
     W.qc2[o] = qc2;
     W.mut[o] = mut;
     // the edge cells this cell is the source of: on each axis at most one (periodic: cell
-    // n-2 serves edge 0 and cell 1 edge n-1; non-periodic: each its own neighbour)
+    // n-2 serves edge 0 and cell 1 edge n-1; non-periodic: each its own neighbour).  The
+    // only cell of a periodic axis of three serves both: mut_needs_edges
     const int c3[3] = {i, j, k};
     int e[3];
     bool z[3] = {false, false, false}, any = false;
@@ -805,6 +806,20 @@ __device__ __forceinline__ void mut_edge_cell(const Geo& G, const Fields<T>& W, 
   const int64_t o = G.at(c[0], c[1], c[2]), src = G.at(s[0], s[1], s[2]);
   W.mut[o] = zero ? T(0) : W.mut[src];
   W.qc2[o] = zero ? T(0) : W.qc2[src];
+}
+
+// Whether k_mut leaves edge cells unwritten: a periodic axis of three cells, whose one
+// interior cell is the source of both its edges (order 2).  k_mut_edges then writes them
+// all; counting both edges in k_mut costs every grid registers (81^3 LES step 502 -> 634 us).
+inline bool mut_needs_edges(const Geo& G) {
+  return (!G.bcx && G.nx == 3) || (!G.bcy && G.ny == 3) || (G.bcz == 0 && G.nz == 3);
+}
+template <class T>
+__global__ void k_mut_edges(Geo G, Fields<T> W) {
+  step_begin();
+  const int64_t n = (int64_t)G.nx * G.ny * G.nz;
+  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n; t += (int64_t)gridDim.x * blockDim.x)
+    mut_edge_cell<T>(G, W, t);
 }
 
 // ---- ghost / boundary-cell fill ------------------------------------------------
