@@ -133,6 +133,20 @@ inline cudaError_t launch_step(void (*kernel)(P...), dim3 grid, dim3 block, size
   return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
 }
 
+// A plain load that stays where it is written: the compiler moves others down to their
+// use, or apart where they stand under a condition (k_prim_mx at 384^3: 791 us with C++
+// loads, 748 with these).
+__device__ __forceinline__ double load_here(const double* p) {
+  double v;
+  asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ float load_here(const float* p) {
+  float v;
+  asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+  return v;
+}
+
 // Padded cell (i, j, k) of a flat index t (x fastest over nx, then ny, then nz).
 __device__ __forceinline__ void cell_of(const Geo& G, int64_t t, int& i, int& j, int& k) {
   i = (int)(t % G.nx);
@@ -227,7 +241,7 @@ __device__ __forceinline__ void prim_mx_cell(const double* Qn, const float* dQ, 
   double q[5];
 #pragma unroll
   for (int l = 0; l < DIM + 2; ++l)
-    q[l] = Qn[o + l * G.vs] + (dQ ? (double)dQ[o + l * G.vs] : 0.0);
+    q[l] = load_here(Qn + o + l * G.vs) + (dQ ? (double)load_here(dQ + o + l * G.vs) : 0.0);
   double v[3];
   prim_store<DIM, VISC, true>(q, jac[(int64_t)j * G.nx + i], W, o, K, v);
 }
@@ -531,11 +545,14 @@ inline dim3 grad_grid(const Geo& G) {
 // SENSOR: the same pass also writes the Ducros sensor of its cells from the +-1
 // neighbours it loads for the gradients (the arithmetic of sensor_of_diffs), so that
 // the primitive pass before it can be the plain per-cell k_prim.  Every neighbour value
-// is loaded once and feeds both.  Bounded to 8 blocks per SM (32 registers; the FP64
-// sensor pass spills 24 B): measured on B200 at 518^3 faster than its 40 registers at
-// 6 blocks per SM, 3.79 against 4.06 ms (this latency-bound pass wants resident warps).
+// is loaded once and feeds both; an axis' loads all stand before its stores, which they
+// may not pass.  Latency-bound: it wants resident warps, 8 blocks per SM (32 registers),
+// but with the FP64 sensor loads in flight, 6 (40 registers, no spills): measured on B200 at
+// 384^3 / 224^3 (ms, ME4) 8 blocks 1.79 / 0.355, 6 blocks 1.49 / 0.304; without the sensor
+// 1.30 / 0.268.
 template <bool SIXTH, class T, bool SENSOR = false>
-__global__ void __launch_bounds__(PLANE_THREADS, 8) k_grad(Geo G, Fields<T> W, Metrics M) {
+__global__ void __launch_bounds__(PLANE_THREADS, SENSOR && sizeof(T) == sizeof(double) ? 6 : 8)
+k_grad(Geo G, Fields<T> W, Metrics M) {
   step_begin();
   const int t = blockIdx.x * PLANE_THREADS + threadIdx.x;
   if (t >= G.nx * G.ny) return;
@@ -560,22 +577,26 @@ __global__ void __launch_bounds__(PLANE_THREADS, 8) k_grad(Geo G, Fields<T> W, M
     const bool fits = c[a] >= HD && c[a] + HD < n[a];
     const T inv = fits ? (T)invd[a][c[a]] : T(0);
     const T sc = sens ? ducros_scale<T>(invd[a], c[a]) : T(0);
-    T d[3];  // (-vel_q(o - st_a) + vel_q(o + st_a)) times the sensor's scale
-    T gq[3] = {};  // stored after the three components' loads: a load may not pass a store
+    T d[3] = {};  // (-vel_q(o - st_a) + vel_q(o + st_a)) times the sensor's scale
+    T gq[3] = {};
+    // all of the axis' loads before its stores: a load may not pass a store
+    if (fits) {
+      T m1[3], p1[3], m2[3], p2[3], m3[3] = {}, p3[3] = {};
 #pragma unroll
-    for (int q = 0; q < 3; ++q) {
-      const T* f = vel[q] + o;
-      d[q] = T(0);
-      if (fits) {
-        const T m1 = f[-st[a]], p1 = f[st[a]];
-        const T m2 = f[-2 * st[a]], p2 = f[2 * st[a]];
-        T m3 = T(0), p3 = T(0);
-        if constexpr (SIXTH) { m3 = f[-3 * st[a]]; p3 = f[3 * st[a]]; }
-        gq[q] = node_deriv_of<SIXTH, T>(m3, m2, m1, p1, p2, p3, inv);
-        if (sens) d[q] = (-m1 + p1) * sc;
-      } else if (sens) {
-        d[q] = (-f[-st[a]] + f[st[a]]) * sc;
+      for (int q = 0; q < 3; ++q) {
+        const T* f = vel[q] + o;
+        m1[q] = f[-st[a]]; p1[q] = f[st[a]];
+        m2[q] = f[-2 * st[a]]; p2[q] = f[2 * st[a]];
+        if constexpr (SIXTH) { m3[q] = f[-3 * st[a]]; p3[q] = f[3 * st[a]]; }
       }
+#pragma unroll
+      for (int q = 0; q < 3; ++q) {
+        gq[q] = node_deriv_of<SIXTH, T>(m3[q], m2[q], m1[q], p1[q], p2[q], p3[q], inv);
+        d[q] = (-m1[q] + p1[q]) * sc;
+      }
+    } else if (sens) {
+#pragma unroll
+      for (int q = 0; q < 3; ++q) d[q] = (-vel[q][o - st[a]] + vel[q][o + st[a]]) * sc;
     }
 #pragma unroll
     for (int q = 0; q < 3; ++q) W.grad[3 * q + a][o] = gq[q];

@@ -63,13 +63,6 @@ template <class T, bool LES, bool SHARE> __host__ __device__ constexpr size_t ym
          (SHARE ? sizeof(T) * me4_terms<LES>() * (YM_R + 2) * YM_C : 0);
 }
 
-// a load that stays where it is written (the compiler would move it down to its use)
-__device__ __forceinline__ double load_early(const double* p) {
-  double v;
-  asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p));
-  return v;
-}
-
 template <int ORDER, int VK, bool LES, class T, bool SHARE>
 __global__ void __launch_bounds__(32 * MARCH_WARPS, ym_minb<T>()) k_march_y(StepArgs<T> A, int seg) {
   step_begin();
@@ -119,7 +112,7 @@ __global__ void __launch_bounds__(32 * MARCH_WARPS, ym_minb<T>()) k_march_y(Step
     double ra[5] = {};  // the cell's accumulator travels while its face is evaluated
     if (cell) {
 #pragma unroll
-      for (int l = 0; l < 5; ++l) ra[l] = load_early(racc + l * G.vs);
+      for (int l = 0; l < 5; ++l) ra[l] = load_here(racc + l * G.vs);
     }
     int off[6];
 #pragma unroll
