@@ -221,6 +221,8 @@ void build_tables(oux_handle* h) {
   K.delta15 = c.visc == OUX_LES && h->G.uni == 7 ? sms_delta15_host(c) : 0.0;
 }
 
+bool uses_grads(const oux_config& c);
+
 Geo make_geo(const oux_config& c) {
   Geo G;
   G.dim = c.dim; G.nx = c.nx; G.ny = c.ny; G.nz = c.dim == 3 ? c.nz : 1; G.g = c.order / 2;
@@ -258,6 +260,7 @@ Geo make_geo(const oux_config& c) {
     for (int i = 1; i < n[a] - 1 && same; ++i) same = std::memcmp(&d[a][i], &d[a][0], sizeof(double)) == 0;
     if (same) G.uni |= 1 << a;
   }
+  G.early = !uses_grads(c) || (int64_t)c.nx * c.ny * c.nz < 1500000;
   G.sx = round_up(c.nx, 4);
   G.plane = G.sx * c.ny;
   G.vs = round_up(G.plane * G.nz, 32);
@@ -534,7 +537,7 @@ int launch_prim_fused(const TQ* q, const TS* src, const Geo& G, Fields<T>& W, ou
   auto kern = k_prim_fused<VISC, MX, TQ, T>;
   static const cudaError_t attr = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (attr != cudaSuccess) return 1;
-  launch_step(kern, prim_fused_grid(G), dim3(PS_TX * PS_TY), smem, s, q, inc, G, W, h->M, h->K);
+  launch_step(G, kern, prim_fused_grid(G), dim3(PS_TX * PS_TY), smem, s, q, inc, G, W, h->M, h->K);
   return cudaPeekAtLastError() == cudaSuccess ? 0 : 1;
 }
 
@@ -569,19 +572,19 @@ int run_stage(oux_handle* h, const TS* src, StepArgs<T> A, cudaStream_t s) {
       // mixed form: Q^(s) = Q^n + FP32 increment (no increment for the first stage)
       const float* dQ = std::is_same<TS, double>::value ? nullptr : reinterpret_cast<const float*>(src);
       if (G.dim == 3) {
-        if (visc) launch_step(k_prim_mx<3, true>, gb, dim3(PLANE_THREADS), 0, s, h->Q, dQ, G, h->Wf, h->M.jac, h->K);
-        else launch_step(k_prim_mx<3, false>, gb, dim3(PLANE_THREADS), 0, s, h->Q, dQ, G, h->Wf, h->M.jac, h->K);
+        if (visc) launch_step(G, k_prim_mx<3, true>, gb, dim3(PLANE_THREADS), 0, s, h->Q, dQ, G, h->Wf, h->M.jac, h->K);
+        else launch_step(G, k_prim_mx<3, false>, gb, dim3(PLANE_THREADS), 0, s, h->Q, dQ, G, h->Wf, h->M.jac, h->K);
       } else {
-        if (visc) launch_step(k_prim_mx<2, true>, gb, dim3(PLANE_THREADS), 0, s, h->Q, dQ, G, h->Wf, h->M.jac, h->K);
-        else launch_step(k_prim_mx<2, false>, gb, dim3(PLANE_THREADS), 0, s, h->Q, dQ, G, h->Wf, h->M.jac, h->K);
+        if (visc) launch_step(G, k_prim_mx<2, true>, gb, dim3(PLANE_THREADS), 0, s, h->Q, dQ, G, h->Wf, h->M.jac, h->K);
+        else launch_step(G, k_prim_mx<2, false>, gb, dim3(PLANE_THREADS), 0, s, h->Q, dQ, G, h->Wf, h->M.jac, h->K);
       }
     } else {
       if (G.dim == 3) {
-        if (visc) launch_step(k_prim<3, true, TS, T>, gb, dim3(PLANE_THREADS), 0, s, src, G, W, h->M.jac, h->K);
-        else launch_step(k_prim<3, false, TS, T>, gb, dim3(PLANE_THREADS), 0, s, src, G, W, h->M.jac, h->K);
+        if (visc) launch_step(G, k_prim<3, true, TS, T>, gb, dim3(PLANE_THREADS), 0, s, src, G, W, h->M.jac, h->K);
+        else launch_step(G, k_prim<3, false, TS, T>, gb, dim3(PLANE_THREADS), 0, s, src, G, W, h->M.jac, h->K);
       } else {
-        if (visc) launch_step(k_prim<2, true, TS, T>, gb, dim3(PLANE_THREADS), 0, s, src, G, W, h->M.jac, h->K);
-        else launch_step(k_prim<2, false, TS, T>, gb, dim3(PLANE_THREADS), 0, s, src, G, W, h->M.jac, h->K);
+        if (visc) launch_step(G, k_prim<2, true, TS, T>, gb, dim3(PLANE_THREADS), 0, s, src, G, W, h->M.jac, h->K);
+        else launch_step(G, k_prim<2, false, TS, T>, gb, dim3(PLANE_THREADS), 0, s, src, G, W, h->M.jac, h->K);
       }
     }
     h->launches++;
@@ -591,11 +594,11 @@ int run_stage(oux_handle* h, const TS* src, StepArgs<T> A, cudaStream_t s) {
     const dim3 gb = plane_grid(G);
     if constexpr (sizeof(T) < sizeof(double)) {
       const float* dQ = std::is_same<TS, double>::value ? nullptr : reinterpret_cast<const float*>(src);
-      if (G.dim == 3) launch_step(k_sensor_mx<3>, gb, dim3(PLANE_THREADS), 0, s, G, h->Q, dQ, h->Wf, h->M);
-      else launch_step(k_sensor_mx<2>, gb, dim3(PLANE_THREADS), 0, s, G, h->Q, dQ, h->Wf, h->M);
+      if (G.dim == 3) launch_step(G, k_sensor_mx<3>, gb, dim3(PLANE_THREADS), 0, s, G, h->Q, dQ, h->Wf, h->M);
+      else launch_step(G, k_sensor_mx<2>, gb, dim3(PLANE_THREADS), 0, s, G, h->Q, dQ, h->Wf, h->M);
     } else {
-      if (G.dim == 3) launch_step(k_sensor<3, T>, gb, dim3(PLANE_THREADS), 0, s, G, W, h->M);
-      else launch_step(k_sensor<2, T>, gb, dim3(PLANE_THREADS), 0, s, G, W, h->M);
+      if (G.dim == 3) launch_step(G, k_sensor<3, T>, gb, dim3(PLANE_THREADS), 0, s, G, W, h->M);
+      else launch_step(G, k_sensor<2, T>, gb, dim3(PLANE_THREADS), 0, s, G, W, h->M);
     }
     h->launches++;
   }
@@ -603,11 +606,11 @@ int run_stage(oux_handle* h, const TS* src, StepArgs<T> A, cudaStream_t s) {
     Timed tm(h, KK_GRAD, s);
     if (G.gk1 > G.gk0) {
       if (sens_in_grad) {
-        if (vk_base(h->vk) == VK_C6) launch_step(k_grad<true, T, true>, grad_grid(G), dim3(PLANE_THREADS), 0, s, G, W, h->M);
-        else launch_step(k_grad<false, T, true>, grad_grid(G), dim3(PLANE_THREADS), 0, s, G, W, h->M);
+        if (vk_base(h->vk) == VK_C6) launch_step(G, k_grad<true, T, true>, grad_grid(G), dim3(PLANE_THREADS), 0, s, G, W, h->M);
+        else launch_step(G, k_grad<false, T, true>, grad_grid(G), dim3(PLANE_THREADS), 0, s, G, W, h->M);
       } else {
-        if (vk_base(h->vk) == VK_C6) launch_step(k_grad<true, T>, grad_grid(G), dim3(PLANE_THREADS), 0, s, G, W, h->M);
-        else launch_step(k_grad<false, T>, grad_grid(G), dim3(PLANE_THREADS), 0, s, G, W, h->M);
+        if (vk_base(h->vk) == VK_C6) launch_step(G, k_grad<true, T>, grad_grid(G), dim3(PLANE_THREADS), 0, s, G, W, h->M);
+        else launch_step(G, k_grad<false, T>, grad_grid(G), dim3(PLANE_THREADS), 0, s, G, W, h->M);
       }
       h->launches++;
     }
@@ -619,12 +622,12 @@ int run_stage(oux_handle* h, const TS* src, StepArgs<T> A, cudaStream_t s) {
       static const cudaError_t attr =
           cudaFuncSetAttribute(k_mut<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       if (attr != cudaSuccess) return fail(OUX_E_CUDA, "SGS viscosity pass: shared memory");
-      launch_step(k_mut<T>, mut_grid(G), dim3(MUT_TX * MUT_TY), smem, s, G, W, h->M, h->K);
+      launch_step(G, k_mut<T>, mut_grid(G), dim3(MUT_TX * MUT_TY), smem, s, G, W, h->M, h->K);
       h->launches++;
     }
     if (mut_needs_edges(G)) {
       Timed tm(h, KK_MUT_EDGES, s);
-      launch_step(k_mut_edges<T>, grid_for((int64_t)G.nx * G.ny * G.nz, 256), dim3(256), 0, s, G, W);
+      launch_step(G, k_mut_edges<T>, grid_for((int64_t)G.nx * G.ny * G.nz, 256), dim3(256), 0, s, G, W);
       h->launches++;
     }
   }
@@ -653,7 +656,7 @@ int ghost(oux_handle* h, T* Q, cudaStream_t s) {
   int64_t n = (int64_t)G.nx * G.ny * G.nz;
   Timed tm(h, KK_GHOST, s);
   const double* Qn = sizeof(T) < sizeof(double) ? h->Q : nullptr;
-  launch_step(k_ghost<T>, grid_for(n / 4 + 1, 256), dim3(256), 0, s, Q, G, h->nv, Qn);
+  launch_step(G, k_ghost<T>, grid_for(n / 4 + 1, 256), dim3(256), 0, s, Q, G, h->nv, Qn);
   h->launches++;
   return OUX_OK;
 }

@@ -63,6 +63,8 @@ struct Geo {
   int uni;                    // bit a: every spacing along axis a is the same double (so are
                               // the inverse spacings), which lets the ME4 sweeps share the
                               // values of a face position between the three faces using it
+  int early;                  // 1: the step's kernels are launched with programmatic stream
+                              // serialisation (launch_step)
   __host__ __device__ int64_t at(int i, int j, int k) const { return (int64_t)k * plane + (int64_t)j * sx + i; }
 };
 
@@ -114,12 +116,17 @@ template <class T> struct StepArgs {
 // set-up hides a launch's latency, 1 to 3 us, which counts on small grids: measured on B200
 // (us per pass) 60^3 inviscid RK4 step 221 -> 184, four 64^3 SLAU-6 steps 1489 -> 1339, 81^3
 // LES step 541 -> 504, ten 513 x 7 steps 430 -> 382.
+// Large 3D grids with gradient fields are launched plainly (Geo::early): their sweeps
+// want most of an SM as shared memory, and blocks set up while the kernel before still
+// holds the SM with another split of it find less room than after it.  us per step, plain /
+// programmatic (mixed ME4, KEEP): 100^3 586 / 577, 128^3 1014 / 1041, 160^3 1856 / 1920, 256^3
+// 6502 / 7574; FP64 Central-6 128^3 1330 / 1302, 256^3 9047 / 9051.
 __device__ __forceinline__ void step_begin() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 template <class... P, class... A>
-inline cudaError_t launch_step(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args) {
+inline cudaError_t launch_step(const Geo& G, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args) {
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
@@ -129,7 +136,7 @@ inline cudaError_t launch_step(void (*kernel)(P...), dim3 grid, dim3 block, size
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = G.early ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
 }
 

@@ -53,9 +53,9 @@ int launch_one(const StepArgs<T>& A, int last, cudaStream_t s) {
     if (A.tmaps) std::memcpy(&maps, static_cast<const unsigned char*>(A.tmaps) + DIR * sizeof(SweepMaps),
                              sizeof(SweepMaps));
     else std::memset(&maps, 0, sizeof(SweepMaps));
-    rc = launch_step(k_sweep_tm<DIM, DIR, ORDER, VK, LES, T, SHARE>, grid, block, smem, s, A, last, maps, A.tmaps ? 1 : 0);
+    rc = launch_step(G, k_sweep_tm<DIM, DIR, ORDER, VK, LES, T, SHARE>, grid, block, smem, s, A, last, maps, A.tmaps ? 1 : 0);
   } else {
-    rc = launch_step(k_sweep<DIM, DIR, ORDER, VK, LES, T, SHARE>, grid, block, smem, s, A, last);
+    rc = launch_step(G, k_sweep<DIM, DIR, ORDER, VK, LES, T, SHARE>, grid, block, smem, s, A, last);
   }
   return rc == cudaSuccess ? 0 : 1;
 }

@@ -196,7 +196,7 @@ int launch_march_y(const StepArgs<T>& A, cudaStream_t s) {
   const int seg = march_split(Ny, 148 * ym_minb<T>() * MARCH_WARPS, (int64_t)groups * Nz, 2.0,
                               [](int c) { return (c + YM_R) / YM_R; });
   const dim3 grid((unsigned)((groups + MARCH_WARPS - 1) / MARCH_WARPS), (unsigned)((Ny + seg - 1) / seg), (unsigned)Nz);
-  return launch_step(kern, grid, dim3(32 * MARCH_WARPS), smem, s, A, seg) == cudaSuccess ? 0 : 1;
+  return launch_step(G, kern, grid, dim3(32 * MARCH_WARPS), smem, s, A, seg) == cudaSuccess ? 0 : 1;
 }
 
 // ---- z sweep -----------------------------------------------------------------------
@@ -350,7 +350,7 @@ int launch_march_z(const StepArgs<T>& A, cudaStream_t s) {
   if (Nz <= 0) return 0;  // an empty part of a split stage
   const int groups = (Nx + 31) / 32, seg = march_split(Nz, 148 * zm_minb<T>() * zm_warps<T>(), (int64_t)groups * Ny, 4.0, [](int c) { return c; });
   const dim3 grid((unsigned)((groups + zm_warps<T>() - 1) / zm_warps<T>()), (unsigned)Ny, (unsigned)((Nz + seg - 1) / seg));
-  return launch_step(kern, grid, dim3(32 * zm_warps<T>()), smem, s, A, seg) == cudaSuccess ? 0 : 1;
+  return launch_step(G, kern, grid, dim3(32 * zm_warps<T>()), smem, s, A, seg) == cudaSuccess ? 0 : 1;
 }
 
 // ---- x sweep ---------------------------------------------------------------------
@@ -485,7 +485,7 @@ int launch_march_x(const StepArgs<T>& A, cudaStream_t s) {
                                            [&](int r) { return ((int64_t)r * E + 31) / 32; }));
   const int warps = (Ny + nrow - 1) / nrow;
   const dim3 grid((unsigned)((warps + MARCH_WARPS - 1) / MARCH_WARPS), (unsigned)Nz, 1);
-  return launch_step(kern, grid, dim3(32 * MARCH_WARPS), smem, s, A, nrow, E) == cudaSuccess ? 0 : 1;
+  return launch_step(G, kern, grid, dim3(32 * MARCH_WARPS), smem, s, A, nrow, E) == cudaSuccess ? 0 : 1;
 }
 
 template <int DIR, int ORDER, int VK, bool LES, class T, bool SHARE>

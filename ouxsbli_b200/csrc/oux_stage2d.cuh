@@ -256,7 +256,7 @@ int launch_stage2d(const StepArgs<T>& A, const void* src, void* dst, double* kee
   if (attr != cudaSuccess) return 1;
   const Geo& G = A.G;
   const dim3 grid((unsigned)((G.nx - 2 * G.gx + S2_TX - 1) / S2_TX), (unsigned)((G.ny - 2 * G.gy + S2_TY - 1) / S2_TY));
-  return launch_step(kern, grid, dim3(S2_THREADS), smem, s, A, src, dst, keep) == cudaSuccess ? 0 : 1;
+  return launch_step(G, kern, grid, dim3(S2_THREADS), smem, s, A, src, dst, keep) == cudaSuccess ? 0 : 1;
 }
 
 template <class T>

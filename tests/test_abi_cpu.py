@@ -231,8 +231,8 @@ def test_step_kernels_wait_first_and_load_plainly():
     which has no order with the wait.  Read from the sources."""
     csrc = HEADER.parents[1] / "ouxsbli_b200" / "csrc"
     text = {p.name: re.sub(r"//[^\n]*", "", p.read_text()) for p in csrc.glob("*.cu*")}
-    launched = {k for t in text.values() for k in re.findall(r"launch_step\(\s*(k_\w+)", t)}
-    launched |= {k for t in text.values() if "launch_step(kern" in t for k in re.findall(r"auto kern = (k_\w+)", t)}
+    launched = {k for t in text.values() for k in re.findall(r"launch_step\(G, (k_\w+)", t)}
+    launched |= {k for t in text.values() if "launch_step(G, kern" in t for k in re.findall(r"auto kern = (k_\w+)", t)}
     assert {"k_prim", "k_prim_fused", "k_grad", "k_mut", "k_ghost", "k_sweep", "k_sweep_tm", "k_march_x", "k_march_y",
             "k_march_z", "k_stage2d"} <= launched
     found = set()
