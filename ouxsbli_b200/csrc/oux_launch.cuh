@@ -10,7 +10,10 @@ template <int DIM, int DIR, int ORDER, int VK, bool LES, class T, bool SHARE = f
 int launch_one(const StepArgs<T>& A, int last, cudaStream_t s) {
   if constexpr (DIM == 3 && sweep_uses_grads<DIM, VK>() && !SHARE) {
     // marching sweeps from the size on where they are the faster ones (march_min_cells)
-    const int64_t cells = (int64_t)(A.G.nx - 2 * A.G.gx) * (A.G.ny - 2 * A.G.gy) * (A.G.sk1 - A.G.sk0);
+    const int64_t Ny = A.G.ny - 2 * A.G.gy, Nz = A.G.sk1 - A.G.sk0;
+    // (for the x march, none if the grid has too few rows)
+    const bool rows = DIR != 0 || (Ny + SWEEP_BR - 1) / SWEEP_BR * SWEEP_BR * Nz >= MARCH_MIN_ROWS;
+    const int64_t cells = rows ? (A.G.nx - 2 * A.G.gx) * Ny * Nz : 0;
     const bool share = VK == VK_ME4 && ((A.G.uni >> DIR) & 1);
     if constexpr (VK == VK_ME4) {
       if (share && cells >= march_min_cells<DIR, T, true>())

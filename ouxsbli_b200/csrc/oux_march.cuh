@@ -167,18 +167,34 @@ __global__ void __launch_bounds__(32 * MARCH_WARPS, ym_minb<T>()) k_march_y(Step
   }
 }
 
+// Warps a march has resident at `blocks` blocks per SM on the device (0: the kernel cannot
+// be launched), asked once per kernel; allows the kernel its shared memory.
+template <class K>
+int march_slots(K kern, int warps, int blocks, size_t smem) {
+  int dev = 0, sms = 0;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+      cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    return 0;
+  return sms * blocks * warps;
+}
+
 // The segment length (rows per warp in the x sweep) of an axis of n cells on `lines` warp
 // lines, by the fewest rounds on the busiest of the resident warps; `start` rounds are
-// what a warp's start costs (its ring is empty).
+// what a warp's start costs (its ring is empty).  For a given number of waves of warps
+// the most segments that fit are the best, so only those are tried.
 template <class F>
 int march_split(int n, int64_t slots, int64_t lines, double start, F rounds) {
   int best = n;
-  double cost = 0.0;
-  for (int p = 1; p <= std::min(n, 256); ++p) {
-    const int seg = (n + p - 1) / p;
-    const int64_t warps = lines * ((n + seg - 1) / seg);
-    const double c = (double)((warps + slots - 1) / slots) * (rounds(seg) + start);
-    if (p == 1 || c < cost) { cost = c; best = seg; }
+  double cost = ((lines + slots - 1) / slots) * (rounds(n) + start);
+  for (int64_t w = 1; w <= 32; ++w) {
+    const int64_t p = std::min<int64_t>(n, w * slots / lines);  // segments
+    if (p < 1) continue;
+    const int seg = (int)((n + p - 1) / p);
+    const int64_t waves = (lines * ((n + seg - 1) / seg) + slots - 1) / slots;
+    const double c = (double)waves * (rounds(seg) + start);
+    if (c < cost) { cost = c; best = seg; }
+    if (p == n) break;
   }
   return best;
 }
@@ -187,14 +203,13 @@ template <int ORDER, int VK, bool LES, class T, bool SHARE>
 int launch_march_y(const StepArgs<T>& A, cudaStream_t s) {
   auto kern = k_march_y<ORDER, VK, LES, T, SHARE>;
   constexpr size_t smem = MARCH_WARPS * ym_warp_smem<T, LES, SHARE>();
-  static const cudaError_t attr = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (attr != cudaSuccess) return 1;
+  static const int slots = march_slots(kern, MARCH_WARPS, ym_minb<T>(), smem);
+  if (!slots) return 1;
   const Geo& G = A.G;
   const int Ny = G.ny - 2 * G.gy, Nz = G.sk1 - G.sk0;
   if (Nz <= 0) return 0;  // an empty part of a split stage
   const int groups = (G.nx - G.gx + YM_C - 1) / YM_C;
-  const int seg = march_split(Ny, 148 * ym_minb<T>() * MARCH_WARPS, (int64_t)groups * Nz, 2.0,
-                              [](int c) { return (c + YM_R) / YM_R; });
+  const int seg = march_split(Ny, slots, (int64_t)groups * Nz, 2.0, [](int c) { return (c + YM_R) / YM_R; });
   const dim3 grid((unsigned)((groups + MARCH_WARPS - 1) / MARCH_WARPS), (unsigned)((Ny + seg - 1) / seg), (unsigned)Nz);
   return launch_step(G, kern, grid, dim3(32 * MARCH_WARPS), smem, s, A, seg) == cudaSuccess ? 0 : 1;
 }
@@ -343,12 +358,13 @@ template <int ORDER, int VK, bool LES, class T, bool SHARE>
 int launch_march_z(const StepArgs<T>& A, cudaStream_t s) {
   auto kern = k_march_z<ORDER, VK, LES, T, SHARE>;
   constexpr size_t smem = zm_warps<T>() * zm_warp_smem<T, LES, SHARE>();
-  static const cudaError_t attr = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (attr != cudaSuccess) return 1;
+  static const int slots = march_slots(kern, zm_warps<T>(), zm_minb<T>(), smem);
+  if (!slots) return 1;
   const Geo& G = A.G;
   const int Nx = G.nx - 2 * G.gx, Ny = G.ny - 2 * G.gy, Nz = G.sk1 - G.sk0;
   if (Nz <= 0) return 0;  // an empty part of a split stage
-  const int groups = (Nx + 31) / 32, seg = march_split(Nz, 148 * zm_minb<T>() * zm_warps<T>(), (int64_t)groups * Ny, 4.0, [](int c) { return c; });
+  const int groups = (Nx + 31) / 32;
+  const int seg = march_split(Nz, slots, (int64_t)groups * Ny, 4.0, [](int c) { return c; });
   const dim3 grid((unsigned)((groups + zm_warps<T>() - 1) / zm_warps<T>()), (unsigned)Ny, (unsigned)((Nz + seg - 1) / seg));
   return launch_step(G, kern, grid, dim3(32 * zm_warps<T>()), smem, s, A, seg) == cudaSuccess ? 0 : 1;
 }
@@ -475,14 +491,13 @@ template <int ORDER, int VK, bool LES, class T, bool SHARE>
 int launch_march_x(const StepArgs<T>& A, cudaStream_t s) {
   auto kern = k_march_x<ORDER, VK, LES, T, SHARE>;
   constexpr size_t smem = MARCH_WARPS * march_x_warp_smem<T, LES, SHARE>();
-  static const cudaError_t attr = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (attr != cudaSuccess) return 1;
+  static const int slots = march_slots(kern, MARCH_WARPS, march_x_minb<T>(), smem);
+  if (!slots) return 1;
   const Geo& G = A.G;
   const int Nx = G.nx - 2 * G.gx, Ny = G.ny - 2 * G.gy, Nz = G.sk1 - G.sk0;
   if (Nz <= 0) return 0;  // an empty part of a split stage
   const int E = std::max(Nx + 1 + (SHARE ? 2 : 0), 32);
-  const int nrow = std::min(16, march_split(Ny, 148 * march_x_minb<T>() * MARCH_WARPS, Nz, 1.5,
-                                           [&](int r) { return ((int64_t)r * E + 31) / 32; }));
+  const int nrow = std::min(16, march_split(Ny, slots, Nz, 1.5, [&](int r) { return ((int64_t)r * E + 31) / 32; }));
   const int warps = (Ny + nrow - 1) / nrow;
   const dim3 grid((unsigned)((warps + MARCH_WARPS - 1) / MARCH_WARPS), (unsigned)Nz, 1);
   return launch_step(G, kern, grid, dim3(32 * MARCH_WARPS), smem, s, A, nrow, E) == cudaSuccess ? 0 : 1;
@@ -505,6 +520,12 @@ int launch_march_dir(const StepArgs<T>& A, cudaStream_t s) {
 //   z mixed: 192^3 400 / 364 (C6), 475 / 380 (ME4); 224^3 479 / 559 and 586 / 584; 256^3
 //     642 / 829 and 756 / 867
 //   z FP64, Central-6 (its viscous rows double the ring): 256^3 1311 / 1207, so it never marches
+// In x a warp takes whole rows, so a grid with few of them leaves the SMs idle whatever its
+// size; MARCH_MIN_ROWS is half the resident warps, in rows as the tiles count them (they
+// work on four at a time).  us per x sweep, march / tile, FP64 Hybrid-6 ME4 and KEEP-6:
+// 600 rows of 1024 67 / 49 and 51 / 41, of 4096 255 / 166 and 180 / 137; 1200 of 1024
+// 88 / 88 and 68 / 74, of 4096 303 / 315 and 244 / 262; 640 x 1 x 640 48 / 94 and 45 / 80.
+constexpr int64_t MARCH_MIN_ROWS = 1184;
 template <int DIR, class T, bool SHARE> constexpr int64_t march_min_cells() {
   constexpr bool mx = sizeof(T) < sizeof(double);
   if (DIR < 2) return mx ? 100000 : 370000;

@@ -193,7 +193,9 @@ def test_fused_2d_mixed(n, bc, scheme, rk):
 # ---- marching sweeps (oux_march.cuh): from 380 000 interior cells (FP64; x and y), 6 000 000 (z, ME4), mixed 100 000 and 11 000 000 ----
 # extents one past, at and short of 32 columns (x, z) and of 8 (y), segments of one row and of
 # odd lengths, axes of 1 to 3 cells, rows longer than a warp's ring
-XY_SIZES = [(33, 109, 107), (31, 113, 110), (512, 28, 27), (95, 3, 1340), (3, 350, 366), (620, 613, 1)]
+# few long rows (x on tiles), one plane of many rows, one line of columns split along y
+XY_SIZES = [(33, 109, 107), (31, 113, 110), (512, 28, 27), (95, 3, 1340), (3, 350, 366), (620, 613, 1),
+            (2048, 14, 14), (330, 1301, 1), (10, 38001, 1)]
 Z_SIZES = [(97, 251, 249), (33, 430, 426), (1, 2457, 2443)]
 
 
