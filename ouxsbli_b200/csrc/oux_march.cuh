@@ -215,8 +215,9 @@ int launch_march_y(const StepArgs<T>& A, cudaStream_t s) {
 }
 
 // ---- z sweep -----------------------------------------------------------------------
-// A warp owns 32 adjacent x-columns of one y row, lane = column, and marches along z over
-// a segment of cells, one face a round.  A lane's stencil, its cp.async copies, the two
+// A warp owns 32 adjacent x-columns of one y row, lane = column (the warps of a block take
+// consecutive such lines, whatever their number in a row), and marches along z over a
+// segment of cells, one face a round.  A lane's stencil, its cp.async copies, the two
 // ME4 positions and the face flux before its current one are its own: no synchronisation
 // at all.  Rows are 256 contiguous bytes of a plane: the y sweep's 8 columns by 4 faces a
 // warp took 12.0 ms here and 16 by 2 took 10.5 (512^3, ME4, FP64; 8.1 this way), every load
@@ -232,12 +233,17 @@ template <class T, bool LES, bool SHARE> __host__ __device__ constexpr size_t zm
          sizeof(T) * 32 * (ZM_CONV * ZM_ROWS + (march_fields<LES>() - ZM_CONV) * zm_aux_rows<SHARE>());
 }
 // warps per block and blocks per SM: 8 (FP64) / 16 (mixed) resident warps; more leave
-// the L1 too small for the copies in flight
+// the L1 too small for the copies in flight.  The mixed Central and LES rings are larger
+// (58 KB a block and more): 3 blocks, 12 warps, fit the 228 KB of an SM.
 template <class T> __host__ __device__ constexpr int zm_warps() { return sizeof(T) == 8 ? 2 : 4; }
-template <class T> __host__ __device__ constexpr int zm_minb() { return 4; }
+constexpr int ZM_MINB = 4;
+template <class T, bool LES, bool SHARE> constexpr int zm_blocks() {
+  constexpr int fit = (int)(228 * 1024 / (zm_warps<T>() * zm_warp_smem<T, LES, SHARE>() + 1024));
+  return fit < ZM_MINB ? fit : ZM_MINB;
+}
 
 template <int ORDER, int VK, bool LES, class T, bool SHARE>
-__global__ void __launch_bounds__(32 * zm_warps<T>(), zm_minb<T>()) k_march_z(StepArgs<T> A, int seg) {
+__global__ void __launch_bounds__(32 * zm_warps<T>(), ZM_MINB) k_march_z(StepArgs<T> A, int seg) {
   step_begin();
   constexpr int DIR = 2, NC = ZM_ROWS, NA = zm_aux_rows<SHARE>();
   constexpr bool MXC = sizeof(T) < sizeof(double);
@@ -245,15 +251,16 @@ __global__ void __launch_bounds__(32 * zm_warps<T>(), zm_minb<T>()) k_march_z(St
   const Geo& G = A.G;
   const int lane = threadIdx.x & 31;
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);  // warp-uniform
-  const int x0 = G.gx + 32 * (blockIdx.x * zm_warps<T>() + warp);
-  if (x0 >= G.nx - G.gx) return;
+  const int groups = (G.nx - 2 * G.gx + 31) / 32, line = blockIdx.x * zm_warps<T>() + warp;
+  const int row = line / groups, x0 = G.gx + 32 * (line - row * groups);
+  if (row >= G.ny - 2 * G.gy) return;
   unsigned char* ws = smraw + warp * zm_warp_smem<T, LES, SHARE>();
   double* ops = reinterpret_cast<double*>(ws) + lane;                       // [operand][32]
   T* conv = reinterpret_cast<T*>(ws + sizeof(double) * 32 * ZM_OPS) + lane;  // [field][NC][32]
   T* aux = conv + ZM_CONV * NC * 32;                                        // [field - 6][NA][32]
-  const int i = x0 + lane, t = G.gy + blockIdx.y;
+  const int i = x0 + lane, t = G.gy + row;
   const bool xok = i < G.nx - G.gx;
-  const int c0 = G.sk0 + blockIdx.z * seg, c1 = min(G.sk1, c0 + seg);  // cells of the segment
+  const int c0 = G.sk0 + blockIdx.y * seg, c1 = min(G.sk1, c0 + seg);  // cells of the segment
   const int64_t col = G.at(i, t, 0);
   const int f0 = c0 - 1;  // the segment's first face
   const int r0 = f0 - 2;  // and first row, in slot 0 of both rings
@@ -358,14 +365,14 @@ template <int ORDER, int VK, bool LES, class T, bool SHARE>
 int launch_march_z(const StepArgs<T>& A, cudaStream_t s) {
   auto kern = k_march_z<ORDER, VK, LES, T, SHARE>;
   constexpr size_t smem = zm_warps<T>() * zm_warp_smem<T, LES, SHARE>();
-  static const int slots = march_slots(kern, zm_warps<T>(), zm_minb<T>(), smem);
+  static const int slots = march_slots(kern, zm_warps<T>(), zm_blocks<T, LES, SHARE>(), smem);
   if (!slots) return 1;
   const Geo& G = A.G;
   const int Nx = G.nx - 2 * G.gx, Ny = G.ny - 2 * G.gy, Nz = G.sk1 - G.sk0;
   if (Nz <= 0) return 0;  // an empty part of a split stage
   const int groups = (Nx + 31) / 32;
   const int seg = march_split(Nz, slots, (int64_t)groups * Ny, 4.0, [](int c) { return c; });
-  const dim3 grid((unsigned)((groups + zm_warps<T>() - 1) / zm_warps<T>()), (unsigned)Ny, (unsigned)((Nz + seg - 1) / seg));
+  const dim3 grid((unsigned)(((int64_t)groups * Ny + zm_warps<T>() - 1) / zm_warps<T>()), (unsigned)((Nz + seg - 1) / seg));
   return launch_step(G, kern, grid, dim3(32 * zm_warps<T>()), smem, s, A, seg) == cudaSuccess ? 0 : 1;
 }
 

@@ -196,7 +196,7 @@ def test_fused_2d_mixed(n, bc, scheme, rk):
 # few long rows (x on tiles), one plane of many rows, one line of columns split along y
 XY_SIZES = [(33, 109, 107), (31, 113, 110), (512, 28, 27), (95, 3, 1340), (3, 350, 366), (620, 613, 1),
             (2048, 14, 14), (330, 1301, 1), (10, 38001, 1)]
-Z_SIZES = [(97, 251, 249), (33, 430, 426), (1, 2457, 2443)]
+Z_SIZES = [(97, 251, 249), (33, 430, 426), (1, 2457, 2443), (70, 301, 287), (24, 509, 493)]
 
 
 @pytest.mark.parametrize("n", XY_SIZES + Z_SIZES)
