@@ -13,6 +13,7 @@
 #include <vector>
 #include "oux.h"
 #include "oux_sweep.cuh"
+#include "oux_stage2d.cuh"
 #include "oux_dispatch.h"
 #include "oux_internal.h"
 
@@ -753,10 +754,24 @@ int run_stage_n(oux_handle* h, int st, cudaStream_t s, int part = 0) {
 // Whether whole steps of a solve run as one kernel per stage (oux_stage2d.cuh): 2D
 // inviscid, a periodic axis having one cell or at least as many as its ghost cells a side
 // (ghost_cell's image of the others' outer ghost cells is itself a ghost cell).
+//
+// Not on long grids a few cells wide, whose 32 x 8 tiles are mostly padding that the
+// fused stage pays for once there are tiles enough to fill the GPU several times: `most`
+// padded cells per cell, by what the fused stage gains on a full tile.  us per step, fused /
+// separate, at padding 8 (100000 x 1): KEEP-6 FP64 138 / 207, SLAU-6 339 / 351, order-4
+// Hybrid 182 / 150; mixed 186 / 163, 364 / 264, 203 / 141; padding 4.6 (7 x 20000): FP64 143 / 228,
+// 424 / 457, 210 / 213, mixed 148 / 171, 335 / 317, 196 / 181; padding 1.9 (17 x 60000) mixed
+// 466 / 532, 918 / 779, 531 / 453; few tiles (30000 x 1, 938) 79 / 88, 137 / 128, 79 / 82.
 bool fused_2d(const oux_handle* h) {
   const Geo& G = h->G;
   auto fits = [&](int n, bool wall) { return wall || n == 2 * G.g + 1 || n >= 3 * G.g; };
-  return G.dim == 2 && h->vk == VK_EULER && fits(G.nx, G.bcx) && fits(G.ny, G.bcy);
+  if (G.dim != 2 || h->vk != VK_EULER || !fits(G.nx, G.bcx) || !fits(G.ny, G.bcy)) return false;
+  const int64_t Nx = G.nx - 2 * G.gx, Ny = G.ny - 2 * G.gy;
+  const int64_t tiles = (Nx + S2_TX - 1) / S2_TX * ((Ny + S2_TY - 1) / S2_TY);
+  const bool keep = h->cfg.scheme == OUX_KEEP;
+  if (tiles <= 1800 || (keep && !h->mixed)) return true;
+  const double most = !h->mixed ? 5.0 : keep ? 8.0 : 1.5;
+  return (double)(tiles * S2_TX * S2_TY) < most * (double)(Nx * Ny);
 }
 
 // nsteps time steps, one kernel per stage.  The stage states alternate between Qs and

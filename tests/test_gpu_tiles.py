@@ -190,6 +190,28 @@ def test_fused_2d_mixed(n, bc, scheme, rk):
         assert np.abs(a[:, l] - b[:, l]).max() <= 2e-6 * np.abs(b).max()
 
 
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("scheme,rk", [("KEEP", 4), ("SLAU", 3)])
+@pytest.mark.parametrize("n", [(60011, 1), (1, 14501), (3, 15001), (17, 58001)])
+def test_long_narrow_2d_steps(n, scheme, rk, precision):
+    """Both routes of a long grid a few cells wide (1876 to 7251 tiles): fused stages for
+    FP64 KEEP, separate passes for the others from the padding on where those are faster."""
+    from ouxsbli_b200.solver import Solver
+    cfg, qj = box2d(n, 6, scheme=scheme, visc="Euler", rk=rk, precision=precision)
+    s = Solver(cfg)
+    s.set_state(qj)
+    before = s.launches()
+    s.step(1)
+    fused = (scheme == "KEEP" and (precision == "fp64" or n == (17, 58001))) or (precision == "fp64" and n == (17, 58001))
+    assert (s.launches() - before == rk) == fused
+    a, b = s.get_state(), oracle.step(cfg, qj, 1)
+    if precision == "fp64":
+        assert np.array_equal(a, b)
+    else:
+        for l in range(4):
+            assert np.abs(a[:, l] - b[:, l]).max() <= 2e-6 * np.abs(b).max()
+
+
 # ---- marching sweeps (oux_march.cuh): from 380 000 interior cells (FP64; x and y), 6 000 000 (z, ME4), mixed 100 000 and 11 000 000 ----
 # extents one past, at and short of 32 columns (x, z) and of 8 (y), segments of one row and of
 # odd lengths, axes of 1 to 3 cells, rows longer than a warp's ring
