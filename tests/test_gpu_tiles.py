@@ -173,14 +173,15 @@ def test_fused_2d_boundaries(n, bc, y_last):
     assert np.array_equal(s.get_state(), oracle.step(cfg, qj, 3))
 
 
+@pytest.mark.parametrize("order", [2, 4, 6])
 @pytest.mark.parametrize("scheme,rk", [("KEEP", 4), ("Hybrid", 3)])
 @pytest.mark.parametrize("n,bc", [((33, 9), (0, 0)), ((40, 1), (0, 0)), ((31, 17), (1, 1))])
-def test_fused_2d_mixed(n, bc, scheme, rk):
+def test_fused_2d_mixed(n, bc, scheme, rk, order):
     """The mixed form: three steps round the increments of 3 rk stages to FP32 (6e-8 of an
     increment that is at most 10 % of the state), and the fluxes to a few FP32 ulps."""
     from ouxsbli_b200.solver import Solver
     rules = {"x_lo": "slip_wall", "y_lo": "noslip_wall"} if bc[0] else None
-    cfg, qj = box2d(n, 6, *bc, boundary=rules, scheme=scheme, visc="Euler", rk=rk, precision="mixed")
+    cfg, qj = box2d(n, order, *bc, boundary=rules, scheme=scheme, visc="Euler", rk=rk, precision="mixed")
     qj = oracle.fill_ghosts(cfg, qj)
     s = Solver(cfg)
     s.set_state(qj)
@@ -212,7 +213,7 @@ def test_long_narrow_2d_steps(n, scheme, rk, precision):
             assert np.abs(a[:, l] - b[:, l]).max() <= 2e-6 * np.abs(b).max()
 
 
-# ---- marching sweeps (oux_march.cuh): from 380 000 interior cells (FP64; x and y), 6 000 000 (z, ME4), mixed 100 000 and 11 000 000 ----
+# ---- marching sweeps (oux_march.cuh): from 370 000 interior cells (FP64; x and y), 6 000 000 (z, ME4), mixed 100 000 and 11 000 000 ----
 # extents one past, at and short of 32 columns (x, z) and of 8 (y), segments of one row and of
 # odd lengths, axes of 1 to 3 cells, rows longer than a warp's ring
 # few long rows (x on tiles), one plane of many rows, one line of columns split along y
@@ -251,8 +252,8 @@ def test_marching_sweeps_stage_combinations(n, rk):
     assert np.array_equal(s.get_state(), oracle.step(cfg, qj, 1))
 
 
-@pytest.mark.parametrize("stencil", ["Central", "ME4Base"])
-@pytest.mark.parametrize("n", [(65, 77, 79), (97, 113, 111)])
+@pytest.mark.parametrize("n,stencil", [((65, 77, 79), "Central"), ((97, 113, 111), "Central"), ((65, 77, 79), "ME4Base"),
+                                       ((97, 113, 111), "ME4Base"), ((182, 184, 183), "ME4Base")])
 def test_marching_sweeps_les(n, stencil):
     cfg, qj = box(n, scheme="SLAU", visc="LES", visc_stencil=stencil)
     a, b = residuals(cfg, qj)
@@ -270,6 +271,59 @@ def test_marching_sweeps_mixed(n, rk):
     a, b = s.get_state(), oracle.step(cfg, qj, 1)
     for l in range(5):
         assert np.abs(a[:, l] - b[:, l]).max() <= 2e-6 * np.abs(b[:, 1:4] if 1 <= l <= 3 else b[:, l]).max()
+
+
+@pytest.mark.parametrize("n,kw", [
+    ((65, 77, 79), dict(scheme="Hybrid", visc="NS")), ((65, 77, 79), dict(scheme="Hybrid", visc="NS", visc_stencil="ME4Base")),
+    ((65, 77, 79), dict(scheme="SLAU", visc="LES")), ((65, 77, 79), dict(scheme="SLAU", visc="LES", visc_stencil="ME4Base")),
+    ((225, 223, 221), dict(scheme="Hybrid", visc="NS")), ((225, 223, 221), dict(scheme="SLAU", visc="LES")),
+    ((225, 223, 221), dict(scheme="SLAU", visc="LES", visc_stencil="ME4Base"))])
+def test_marching_sweeps_mixed_switches(n, kw):
+    """Mixed residuals of the schemes that switch (sensor threshold, limiters, the HRSLAU2
+    and SMS switches): a face whose switch argument lies within FP32 rounding of its
+    threshold may take the other side.  An argument spread over a range of order one falls
+    that close with probability about 1e-6 a switch; with some ten switches on the 6 faces
+    of a cell fewer than 1e-4 of the cells may differ by more than rounding."""
+    cfg, qj = box(n, precision="mixed", **kw)
+    a, b = residuals(cfg, qj)
+    far = np.zeros(a[:, 0].shape, bool)
+    for l in range(5):
+        far |= ~(np.abs(a[:, l] - b[:, l]) <= 2e-6 * np.abs(qj[:, l]).max())
+    assert far.mean() <= 1e-4
+
+
+def test_marching_and_tile_parts_of_a_z_slab():
+    """Two z slabs of 48 planes: a stage's interior part marches (387 072 cells), the parts
+    next to its ends take tiles; the undivided solve marches throughout.  Same bits."""
+    from ouxsbli_b200.slabs import LocalSlabs
+    from ouxsbli_b200.solver import Solver
+    cfg, qj = box((96, 96, 96), scheme="Hybrid", visc="NS", visc_stencil="ME4Base")
+    s = Solver(cfg)
+    s.set_state(qj)
+    s.step(2)
+    slabs = LocalSlabs(cfg, 2, "cuda:0")
+    slabs.set_state(qj)
+    slabs.step(2)
+    g = cfg.g
+    assert np.array_equal(slabs.get_state()[:, :, :, g:-g], s.get_state()[:, :, :, g:-g])
+    slabs.close()
+
+
+@pytest.mark.parametrize("n,stencil", [((97, 115, 111), "Central"), ((97, 115, 111), "ME4Base"), ((225, 225, 223), "Central"),
+                                       ((225, 225, 223), "ME4Base")])
+def test_marching_sweeps_mixed_walls(n, stencil):
+    """Mixed marches between walls (KEEP: no switches), held as the periodic ones."""
+    from helpers import wall_box
+    from ouxsbli_b200.solver import Solver
+    cfg, qj, _ = wall_box(*n, 6, {"y_lo": "noslip_wall", "y_hi": "noslip_wall", "z_lo": "slip_wall", "z_hi": "noslip_wall"},
+                          bc_z=1, scheme="KEEP", visc="NS", visc_stencil=stencil, precision="mixed")
+    qj = oracle.fill_ghosts(cfg, qj)
+    s = Solver(cfg)
+    s.set_state(qj)
+    x = slice(cfg.g - 1, 1 - cfg.g)  # the interior of the periodic axis
+    a, b = s.rhs()[x], oracle.rhs(cfg, qj)[x]
+    for l in range(5):
+        assert np.abs(a[:, l] - b[:, l]).max() <= 2e-6 * np.abs(qj[:, 1:4] if 1 <= l <= 3 else qj[:, l]).max()
 
 
 @pytest.mark.parametrize("stencil,visc", [("Central", "NS"), ("ME4Base", "NS"), ("Central", "LES")])
