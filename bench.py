@@ -552,8 +552,21 @@ ALG_CELL = {"prim": 96.0, "sensor": 32.0, "prim_sensor": 104.0, "grad": 104.0,
 # kernel kinds of oux_profile_read (enum KernelKind of oux_api.cu); prim_sensor: the 3D
 # pass that writes the primitive fields and the Ducros sensor (the mixed form's sensor
 # schemes); grad: the node velocity gradients (Central-4/6 and ME4 viscous stencils), and
-# in FP64 the Ducros sensor too
-KINDS = ["prim", "sensor", "sgs", "sgs_edges", "sweep_x", "sweep_y", "sweep_z", "ghost", "prim_sensor", "grad"]
+# in FP64 the Ducros sensor too; stage2d: a whole stage of a 2D inviscid solve
+KINDS = ["prim", "sensor", "sgs", "sgs_edges", "sweep_x", "sweep_y", "sweep_z", "ghost", "prim_sensor", "grad",
+         "stage2d"]
+
+
+def sweep_digest():
+    """Digest of the sweep kernels' sources and launch rules, comments and spaces apart: a
+    captured figure is of the kernels that run only while this is the same."""
+    import hashlib
+    import re
+    h = hashlib.sha256()
+    for f in ("oux_march.cuh", "oux_sweep.cuh", "oux_launch.cuh"):
+        with open(os.path.join(ROOT, "ouxsbli_b200", "csrc", f)) as src:
+            h.update("".join(re.sub(r"//[^\n]*", "", src.read()).split()).encode())
+    return h.hexdigest()[:16]
 
 
 def read_profile(h):
@@ -572,21 +585,24 @@ def roofline_of(args, per_kernel, cells, ms_per_step, peaks):
     peak = float(peaks.get("hbm_gbs", 6650.0))
     dom = max(per_kernel, key=lambda k: per_kernel[k]["share"]) if per_kernel else None
     achieved = ALG_CELL.get(dom, 0.0) * cells / (per_kernel[dom]["avg_ms"] / 1e3) / 1e9 if dom else 0.0
-    # ncu figures of the same kernels on a small case of the same physics (profiles/):
-    # DRAM bytes per interior cell of one launch, scaled by the cells of one launch here,
-    # and the FP64-pipe utilisation
+    # ncu figures of the same kernels (profiles/): DRAM bytes per interior cell of one
+    # launch, scaled by the cells of one launch here, and the FP64-pipe utilisation; none
+    # if the sweeps have changed since they were captured, or the grid is another
     traffic, prof = None, {}
     try:
-        prof = json.load(open(os.path.join(ROOT, "profiles", "sweep_traffic.json"))).get(args.workload, {})
+        with open(os.path.join(ROOT, "profiles", "sweep_traffic.json")) as f:
+            prof = json.load(f).get(args.workload, {})
+        if prof.get("sweep_digest") != sweep_digest() or prof.get("interior_cells") != cells:
+            prof = {"source": "no capture of the present sweeps on this grid"}
         if dom in prof.get("dram_bytes_per_interior_cell", {}):
             traffic = prof["dram_bytes_per_interior_cell"][dom] * cells
-    except Exception:
+    except (OSError, ValueError):
         pass
     step_achieved = ALG_BYTES_PER_CELL_STEP * cells / (ms_per_step / 1e3) / 1e9
     return {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
             "traffic": traffic, "kernel": dom,
             "alg_bytes_per_launch": f"{ALG_CELL.get(dom, 0.0):.1f} B x {cells} interior cells "
-                                    "(per-kernel table in DESIGN.md; mean over the 3 RK3 stages)",
+                                    "(fields and state read or written once; mean over the 3 RK3 stages)",
             "traffic_source": prof.get("source"), "fp64_pipe_pct_ncu": prof.get("fp64_pipe_pct"),
             "peak_source": "measured" if "hbm_gbs" in peaks else "fallback",
             "dominant_kernel": dom, "per_kernel": per_kernel,

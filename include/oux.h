@@ -263,10 +263,10 @@ int oux_status(oux_handle* h, int32_t* fault_bits);
 
 /* Per-kernel timing for measurement tools: while enabled, every launch is
  * bracketed by CUDA events on its stream; oux_profile_read synchronizes and
- * returns, per kernel kind (0 prim, 1 sensor, 2 sgs, 3 sgs edges, 4 x sweep,
- * 5 y sweep, 6 z sweep, 7 ghost fill, 8 primitives + sensor, 9 velocity gradients,
- * 10 fused 2D stage), the summed milliseconds and launch
- * counts since the last oux_profile call.  No reference counterpart (the
+ * returns, per kernel kind (0 prim, 1 sensor, 2 sgs, 3 sgs edges (grids with
+ * a periodic axis of three cells), 4 x sweep, 5 y sweep, 6 z sweep, 7 ghost fill,
+ * 8 primitives + sensor, 9 velocity gradients, 10 fused 2D stage), the summed
+ * milliseconds and launch counts since the last oux_profile call.  No reference counterpart (the
  * reference is profiled externally with ncu/nsys scripts). */
 int oux_profile(oux_handle* h, int32_t enable);
 int oux_profile_read(oux_handle* h, double* ms, int64_t* count, int32_t nkinds);

@@ -556,7 +556,7 @@ int run_stage(oux_handle* h, const TS* src, StepArgs<T> A, cudaStream_t s) {
   // takes the fused primitive + sensor pass (the mixed form's sensor from FP64 velocities)
   const bool sens_in_grad = sens && W.grad[0] != nullptr && sizeof(T) == sizeof(double);
   if (G.dim == 3 && sens && !sens_in_grad) {
-    // primitives and sensor in one z-marching pass
+    // primitives and sensor in one pass over tiles
     Timed tm(h, KK_PRIM_FUSED, s);
     int rc;
     if constexpr (sizeof(T) < sizeof(double)) {

@@ -1,11 +1,11 @@
 // Kernels of one explicit stage on the ghost-padded SoA layout.
 //
-// Per stage (3D): prim -> [sensor] -> [SGS mut/qc2 + their edge copy] ->
+// Per stage (3D): prim [+ sensor] -> [gradients + sensor] -> [SGS mut/qc2 with their edges] ->
 //   x sweep (faces -> dt*S*dE into Racc) -> y sweep (+= dt*S*dF) ->
 //   z sweep (+= dt*S*dG, then the RK combination) -> ghost fill.
-// Face fluxes never touch HBM: each sweep block computes the 2*ORDER/2 + 32
-// cell tile of its pencil rows into shared memory, evaluates every face of the
-// tile once, and differences neighbouring faces in shared memory.
+// Face fluxes never touch HBM: a sweep evaluates the faces of a tile in shared memory
+// (oux_sweep.cuh), or of the rows its warps march along (oux_march.cuh), and differences
+// neighbouring ones there.  2D inviscid stages are one kernel (oux_stage2d.cuh).
 #pragma once
 #include <cstdint>
 #include <utility>

@@ -13,11 +13,11 @@
 // them.  Measured on B200 at 512^3 (Hybrid-6 / ME4, FP64, ms per sweep x / y / z): tiles
 // of one block with barriers 8.8 / 9.5 / 9.8; blocks of 8 warps marching a shared ring,
 // three barriers a chunk, y / z 8.6 / 9.1; these 5.1-5.8 / 6.3-6.6 / 8.1 (the clock falls under
-// the power cap as they get faster).  What bounds them: instruction issue and the FP64
-// pipe in x (59 % and 46 % of peak, ncu at 161 x 143 x 117), L1 line slots and load latency
-// in y and z (FP64 pipe 42 %).  Resident warps are limited by what the rings leave of L1:
-// copies in flight need its lines (y 8.2 ms at 16 warps and 220 KB of shared memory, 6.3 at
-// 12 and 165 KB; z 10.2 at 10 and 197 KB, 8.1 at 8 and 178 KB).
+// the power cap as they get faster).  What bounds them (ncu at 184^3, x / y / z): L1 (88 / 86 /
+// 65 % busy: the rings' reads and cp.async lines), instruction issue (54 / 42 / 48 %) and the FP64 pipe (45 / 38 / 40 %), with
+// load latency in y (2.2 long-scoreboard stalls an issue).  Resident warps are limited by
+// what the rings leave of L1: copies in flight need its lines (y 8.2 ms at 16 warps and 220 KB
+// of shared memory, 6.3 at 12 and 165 KB; z 10.2 at 10 and 197 KB, 8.1 at 8 and 178 KB).
 #pragma once
 #include <algorithm>
 #include "oux_sweep.cuh"
@@ -50,13 +50,7 @@ __device__ __forceinline__ void march_fields_of(const StepArgs<T>& A, CP cp) {
 // plane, over a segment of the y axis; lane = (column, face), YM_R faces a chunk.
 constexpr int YM_C = 8, YM_R = 4;
 constexpr int YM_RING = 14;  // rows f-2 .. f+3 of a chunk's and the next one's faces (13); even: 16 (8-byte) banks
-#ifndef YB
-#define YB 6
-#endif
-#ifndef YBF
-#define YBF 7
-#endif
-template <class T> __host__ __device__ constexpr int ym_minb() { return sizeof(T) == 8 ? YB : YBF; }
+template <class T> __host__ __device__ constexpr int ym_minb() { return sizeof(T) == 8 ? 6 : 7; }
 
 template <class T, bool LES, bool SHARE> __host__ __device__ constexpr size_t ym_warp_smem() {
   return sizeof(double) * 5 * YM_C + sizeof(T) * march_fields<LES>() * YM_RING * YM_C +
@@ -518,15 +512,33 @@ int launch_march_dir(const StepArgs<T>& A, cudaStream_t s) {
 }
 
 // Interior cells from which a direction's sweep marches; below, the tile sweeps of
-// oux_sweep.cuh give more blocks.  Measured on B200, us per sweep, march / tile:
-//   x, y FP64 (Hybrid-6 ME4): 64^3 33 / 29 and 35 / 32; 72^3 38 / 43 and 41 / 50; 144^3
-//     194 / 236 and 188 / 260; 256^3 752 / 1122 and 843 / 1205
-//   x, y mixed (SLAU-6 LES): 48^3 12.7 / 15.7 and 14.7 / 16.6; 80^3 30 / 41 and 33 / 41; 128^3
-//     95 / 131 and 86 / 126 (below 48^3 no gain)
-//   z FP64, shared ME4 positions: 176^3 473 / 452; 192^3 533 / 543; 256^3 1003 / 1245
-//   z mixed: 192^3 400 / 364 (C6), 475 / 380 (ME4); 224^3 479 / 559 and 586 / 584; 256^3
-//     642 / 829 and 756 / 867
-//   z FP64, Central-6 (its viscous rows double the ring): 256^3 1311 / 1207, so it never marches
+// oux_sweep.cuh give more blocks.  Measured on B200 on cubes, us per sweep, march / tile:
+//   FP64          64^3     72^3     96^3     128^3     176^3     192^3     256^3
+//   x KEEP ME4    21 / 23  25 / 35  46 / 64  96 / 137  252 / 348 274 / 430 627 / 996
+//   x Hybrid ME4  31 / 28  37 / 41  68 / 76  157 / 158 352 / 402 367 / 493 774 / 1124
+//   x SLAU C6     32 / 29  37 / 42  72 / 78  162 / 163 392 / 424 404 / 515 850 / 1187
+//   x Hybrid ME4, stretched axes (positions not shared)
+//                 33 / 28  39 / 40  81 / 76  172 / 157 409 / 397 433 / 490 872 / 1107
+//   x KEEP C6 walled in y
+//                 21 / 23  26 / 35  51 / 64  104 / 131 263 / 330 283 / 407 652 / 940
+//   y Hybrid ME4  34 / 31  40 / 46  76 / 81  134 / 172 298 / 446 389 / 532 863 / 1208
+//   y KEEP C6     22 / 23  26 / 35  54 / 60  90 / 129  210 / 343 273 / 408 608 / 956
+//   z KEEP ME4    22 / 25  32 / 39  53 / 68  116 / 148 285 / 397 329 / 473 787 / 1105
+//   z Hybrid ME4  40 / 30  61 / 47  96 / 82  214 / 175 477 / 454 540 / 545 1026 / 1248
+//   z SLAU ME4    39 / 32  58 / 50  93 / 86  209 / 186 496 / 492 553 / 587 1139 / 1359
+//   z Hybrid C6   42 / 29  64 / 45  108 / 79 244 / 170 573 / 440 642 / 528 1330 / 1209
+//   z Hybrid ME4 walled in y
+//                 43 / 29  60 / 47  124 / 76 327 / 165 864 / 433 979 / 515 1384 / 1201
+//   mixed         40^3     48^3     64^3     96^3      160^3     224^3     256^3
+//   x Hybrid C6   13 / 13  13 / 16  23 / 21  49 / 54   172 / 218 418 / 566 526 / 834
+//   x LES C6      13 / 13  13 / 16  21 / 21  44 / 58   166 / 242 418 / 647 582 / 958
+//   y LES ME4     13 / 15  17 / 15  23 / 21  52 / 54   166 / 200 400 / 539 584 / 782
+//   z Hybrid C6   17 / 14  21 / 16  25 / 22  60 / 56   212 / 218 548 / 560 641 / 831
+//   z Hybrid ME4  17 / 15  20 / 16  27 / 23  60 / 59   228 / 228 538 / 585 758 / 870
+//   z KEEP C6     13 / 12  14 / 13  17 / 18  37 / 48   146 / 188 380 / 494 523 / 747
+// so the FP64 z march is for shared ME4 positions alone (the viscous rows of Central-6, and
+// of walled grids, double its ring), from where it pays for SLAU faces too; FP64 x marches
+// of faces that mix KEEP and SLAU stay within 10 % of the tiles either way up to 176^3.
 // In x a warp takes whole rows, so a grid with few of them leaves the SMs idle whatever its
 // size; MARCH_MIN_ROWS is half the resident warps, in rows as the tiles count them (they
 // work on four at a time).  us per x sweep, march / tile, FP64 Hybrid-6 ME4 and KEEP-6:

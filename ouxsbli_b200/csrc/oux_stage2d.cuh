@@ -2,11 +2,12 @@
 // tile and its halo, the x and y face fluxes, the stage combination, and the ghost /
 // boundary cells of the cells it writes.
 //
-// Measured on B200 (us, before -> after): 513 x 7 shock tube, SLAU-6 RK3, ten steps 1085 -> 430;
-// 252^2 vortex, KEEP-6 RK4, ten steps 901 -> 328; 64 vortices of 64^2 to 512^2 in one batched step
-// 2115 -> 1002 (FP64) and 1599 -> 980 (mixed).  What bounds it: load latency and barriers
-// at small grids, on large ones the load of a block's tile, which only the two other
-// resident blocks hide (the combination's operands are fetched during the fluxes: without
+// Measured on B200 (us, separate passes -> this): 513 x 7 shock tube, SLAU-6 RK3, ten steps
+// 1085 -> 382; 252^2 vortex, KEEP-6 RK4, ten steps 901 -> 334; 64 vortices of 64^2 to 512^2 in one
+// batched step 2115 -> 968 (FP64) and 1599 -> 966 (mixed).  What bounds it: load latency and
+// barriers at small grids; on large ones L1 (73 % busy in FP64, 63 % mixed, at 2048^2) and
+// latency that the two other resident blocks have to hide (2.6 long-scoreboard and 1.4
+// barrier stalls an issue; the combination's operands are fetched during the fluxes: without
 // that the batched step took 2883).
 //
 // A 2D stage as separate passes (primitives, sensor, two sweeps, ghost fill) is bound by

@@ -1336,7 +1336,10 @@ template <int DIM, int VK> __host__ __device__ constexpr bool sweep_uses_grads()
 // TMA tile layout).  Measured on B200 at 512^3 (Hybrid-6 / ME4, ms per launch, TMA
 // against cp.async): x 8.12 / 8.18 (FP64) and 5.52 / 5.48 (mixed); y 8.74 / 8.80 and
 // 4.89 / 5.30; z 9.46 / 9.11 and 6.39 / 6.24, where a box is 13 rows from 13 planes
-// 2 MB apart; so z keeps cp.async.
+// 2 MB apart; so z keeps cp.async.  At the sizes where the x and y sweeps still work on
+// tiles (march_min_cells) TMA gains nothing: us per step, TMA / cp.async, FP64 Hybrid ME4
+// 32^3 142.6 / 139.6, 48^3 192.5 / 191.0, 64^3 292.0 / 292.9; KEEP C6 32^3 101.4 / 98.6, 64^3
+// 223.3 / 223.3; mixed KEEP C6 32^3 80.5 / 75.7, LES C6 186.0 / 179.5.
 template <int DIM, int DIR, int VK> __host__ __device__ constexpr bool sweep_tma() {
   return DIR <= 1 && sweep_uses_grads<DIM, VK>();
 }
